@@ -89,7 +89,7 @@ struct SceneData {
   DevBuf faces, tri, box_lo, box_hi, scene_ord;
   bool grid_ok = false;
   ffb_grid_info info{};
-  DevBuf cell_start, cell_fill, ref_tri, ref_rec, empty_dist, cell_rec;
+  DevBuf cell_start, cell_fill, ref_tri, ref_rec, face_rec, empty_dist, cell_rec;
 };
 
 }  // namespace
@@ -210,7 +210,8 @@ void release(ffb_ctx* c, DevBuf& b)
 void release_scene(ffb_ctx* c, SceneData& s)
 {
   DevBuf* bufs[] = {&s.faces,      &s.tri,     &s.box_lo,  &s.box_hi,  &s.scene_ord,
-                    &s.cell_start, &s.cell_fill, &s.ref_tri, &s.ref_rec, &s.empty_dist, &s.cell_rec};
+                    &s.cell_start, &s.cell_fill, &s.ref_tri, &s.ref_rec, &s.face_rec, &s.empty_dist,
+                    &s.cell_rec};
   for (DevBuf* b : bufs)
     release(c, *b);
   s.n_faces = -1;
@@ -285,21 +286,50 @@ int grid_blocks(long long n, int threads, int max_blocks = 1 << 20)
   return (int)std::max<long long>(1, std::min<long long>(b, max_blocks));
 }
 
+// Box and cells of a grid in double, as the rays' float grid coordinates see
+// them (cell size 1 / the float inverse).
+TestGeom test_geom(const ffb_grid_info& I)
+{
+  TestGeom t;
+  double d2 = 0.0;
+  t.reach = 0.0;
+  for (int a = 0; a < 3; ++a) {
+    t.lo[a] = I.lo[a];
+    t.cs[a] = 1.0 / (double)(1.f / I.cell[a]);
+    const double e = (double)I.hi[a] - (double)I.lo[a];
+    d2 += e * e;
+    t.reach = std::max(t.reach, std::max(std::fabs((double)I.lo[a]), std::fabs((double)I.hi[a])));
+  }
+  t.size = std::sqrt(d2);
+  return t;
+}
+
 GridView make_view(SceneData& s)
 {
   GridView g;
   const ffb_grid_info& I = s.info;
   g.lo = make_float3(I.lo[0], I.lo[1], I.lo[2]);
-  g.hi = make_float3(I.hi[0], I.hi[1], I.hi[2]);
-  g.cs = make_float3(I.cell[0], I.cell[1], I.cell[2]);
   g.inv_cs = make_float3(1.f / I.cell[0], 1.f / I.cell[1], 1.f / I.cell[2]);
+  g.nf = make_float3((float)I.nx, (float)I.ny, (float)I.nz);
+  const auto bias = [&](float ics) {
+    const float e = 0.25f * I.margin * ics;
+    return e < 0.25f ? e : 0.25f;  // also for a NaN of an infinite box
+  };
+  g.eps = make_float3(bias(g.inv_cs.x), bias(g.inv_cs.y), bias(g.inv_cs.z));
   g.nx = I.nx;
-  g.ny = I.ny;
-  g.nz = I.nz;
-  g.slack = 2.f * I.margin;
+  g.nxy = I.nx * I.ny;
+  g.nxm = I.nx - 1;
+  g.nym = (I.ny - 1) * g.nx;
+  g.nzm = (I.nz - 1) * g.nxy;
+  g.slack = 2.5f * I.margin;
+  g.tie = 3.5f * I.margin;
+  g.near_err = 0.25f * I.margin;
+  const TestGeom t = test_geom(I);
+  g.inv_size = (float)(1.25 / t.size);
   g.ref_tri = dptr<int32_t>(s.ref_tri);
-  g.ref_rec = dptr<TriRec>(s.ref_rec);
-  g.cell_rec = dptr<uint2>(s.cell_rec);
+  g.ref_rec = dptr<TestRec>(s.ref_rec);
+  g.tri = dptr<TriRec>(s.tri);
+  g.cell_rec = dptr<uint2>(s.cell_rec) + cell_pad(I.nx, I.ny);
   return g;
 }
 
@@ -524,8 +554,11 @@ int grid_build(ffb_ctx* c, SceneData& s, const ffb_grid_params* params)
   // with the reference total
   FFB_TRY(ensure(c, c->live_count, sizeof(uint32_t)));
   FFB_CUDA(cudaMemsetAsync(c->live_count.ptr, 0, sizeof(uint32_t), c->stream));
-  k_count_live<<<grid_blocks(s.n_faces, 256), 256, 0, c->stream>>>(dptr<float4>(s.box_lo), dptr<float4>(s.box_hi),
-                                                                  s.n_faces, dptr<uint32_t>(c->live_count));
+  FFB_TRY(ensure(c, s.face_rec, sizeof(TestRec) * (size_t)s.n_faces));
+  k_face_test<<<grid_blocks(s.n_faces, 128), 128, 0, c->stream>>>(dptr<float4>(s.box_lo), dptr<float4>(s.box_hi),
+                                                                 dptr<TriRec>(s.tri), s.n_faces, test_geom(I),
+                                                                 dptr<TestRec>(s.face_rec),
+                                                                 dptr<uint32_t>(c->live_count));
   FFB_CUDA(cudaGetLastError());
   uint32_t total = 0, live = 0;
   FFB_CUDA(cudaMemcpyAsync(&total, dptr<uint32_t>(s.cell_start) + n_cells, sizeof total, cudaMemcpyDeviceToHost,
@@ -541,9 +574,9 @@ int grid_build(ffb_ctx* c, SceneData& s, const ffb_grid_params* params)
                                          dptr<int32_t>(s.ref_tri));
   k_cell_sort<<<grid_blocks(n_cells, 128), 128, 0, c->stream>>>(dptr<uint32_t>(s.cell_start), (int)n_cells,
                                                                 dptr<int32_t>(s.ref_tri));
-  FFB_TRY(ensure(c, s.ref_rec, sizeof(TriRec) * (size_t)std::max<uint32_t>(total, 1)));
-  k_ref_gather<<<grid_blocks(total, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-      dptr<int32_t>(s.ref_tri), total, dptr<TriRec>(s.tri), dptr<TriRec>(s.ref_rec));
+  FFB_TRY(ensure(c, s.ref_rec, sizeof(TestRec) * (size_t)std::max<uint32_t>(total, 1)));
+  k_ref_gather<<<grid_blocks(4ll * total, 256, c->n_sm * 16), 256, 0, c->stream>>>(
+      dptr<int32_t>(s.ref_tri), total, dptr<TestRec>(s.face_rec), dptr<TestRec>(s.ref_rec));
   FFB_CUDA(cudaGetLastError());
   if (I.skip_empty) {
     // one byte per cell and octant; passes along x, y, z double the octants
@@ -556,9 +589,10 @@ int grid_build(ffb_ctx* c, SceneData& s, const ffb_grid_params* params)
                                                                                          I.nz, axis);
     FFB_CUDA(cudaGetLastError());
   }
-  FFB_TRY(ensure(c, s.cell_rec, sizeof(uint2) * (size_t)n_cells));
+  const long long pad = cell_pad(I.nx, I.ny);
+  FFB_TRY(ensure(c, s.cell_rec, sizeof(uint2) * (size_t)(n_cells + 2 * pad)));
   k_cell_rec<<<grid_blocks(n_cells, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-      dptr<uint32_t>(s.cell_start), I.skip_empty ? dptr<uint8_t>(s.empty_dist) : nullptr, n_cells,
+      dptr<uint32_t>(s.cell_start), I.skip_empty ? dptr<uint8_t>(s.empty_dist) : nullptr, n_cells, pad,
       dptr<uint2>(s.cell_rec));
   FFB_CUDA(cudaGetLastError());
   I.n_refs = total;
@@ -643,17 +677,16 @@ int check_counts(int n_faces, const int32_t* front, const int32_t* rear, long lo
 #endif
 
 // The timed kernel variant (no counters, matrix sink) for each launch shape.
-template <bool kSkip, bool kHash, int... S>
+template <bool kHash, int... S>
 void (*shaped_kernel(int shape, std::integer_sequence<int, S...>))(TraceParams)
 {
-  static void (*const table[])(TraceParams) = {k_form_factors<kSkip, false, kHash, false, S>...};
+  static void (*const table[])(TraceParams) = {k_form_factors<false, kHash, false, S>...};
   return table[shape];
 }
 
 // Occupancy-sized persistent launch of the fused kernel for p.n_chunks
 // chunks, in the context's launch shape (the counter and radiance variants
 // always take shape 0).
-template <bool kSkip>
 int launch_fused(ffb_ctx* c, const TraceParams& p, bool timed, cudaStream_t stream = nullptr, int shape = -1)
 {
   if (!stream)
@@ -663,13 +696,13 @@ int launch_fused(ffb_ctx* c, const TraceParams& p, bool timed, cudaStream_t stre
   bool hash = (unsigned long long)p.scene.n_cols * (unsigned long long)p.scene.n_cols < FFB_DIRECT_MIN_WORDS;
   void (*kern)(TraceParams);
   if (p.stats)
-    kern = hash ? k_form_factors<kSkip, true, true> : k_form_factors<kSkip, true, false>;
+    kern = hash ? k_form_factors<true, true> : k_form_factors<true, false>;
   else if (hash)
-    kern = shaped_kernel<kSkip, true>(shape, std::make_integer_sequence<int, kNumShapes>{});
+    kern = shaped_kernel<true>(shape, std::make_integer_sequence<int, kNumShapes>{});
   else
-    kern = shaped_kernel<kSkip, false>(shape, std::make_integer_sequence<int, kNumShapes>{});
+    kern = shaped_kernel<false>(shape, std::make_integer_sequence<int, kNumShapes>{});
   if (p.power) {  // radiance sink: no matrix, no histogram
-    kern = p.stats ? k_form_factors<kSkip, true, false, true> : k_form_factors<kSkip, false, false, true>;
+    kern = p.stats ? k_form_factors<true, false, true> : k_form_factors<false, false, true>;
     hash = false;
   }
   const size_t smem = hash ? kHashSmem : 0;
@@ -879,7 +912,8 @@ extern "C" int ffb_grid_export(ffb_ctx* c, uint32_t* cell_rec, int32_t* ref_tri)
     return fail(FFB_ERR_NO_GRID, "no grid built");
   const size_t n_cells = (size_t)s.info.nx * s.info.ny * s.info.nz;
   if (cell_rec)
-    FFB_CUDA(cudaMemcpyAsync(cell_rec, s.cell_rec.ptr, sizeof(uint2) * n_cells, cudaMemcpyDefault, c->stream));
+    FFB_CUDA(cudaMemcpyAsync(cell_rec, dptr<uint2>(s.cell_rec) + cell_pad(s.info.nx, s.info.ny),
+                             sizeof(uint2) * n_cells, cudaMemcpyDefault, c->stream));
   if (ref_tri && s.info.n_refs > 0)
     FFB_CUDA(cudaMemcpyAsync(ref_tri, s.ref_tri.ptr, sizeof(int32_t) * (size_t)s.info.n_refs, cudaMemcpyDefault,
                              c->stream));
@@ -961,7 +995,7 @@ int cast_impl(ffb_ctx* c, const float* rays6, long long n_rays, int32_t* hit_fac
     GridView g = make_view(s);
     FFB_TRY(ensure(c, c->ray_cursor, sizeof(unsigned long long)));
     FFB_CUDA(cudaMemsetAsync(c->ray_cursor.ptr, 0, sizeof(unsigned long long), c->stream));
-    auto kern = s.info.skip_empty ? k_cast<true> : k_cast<false>;
+    auto kern = k_cast;
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const int blocks = grid_blocks(n_rays, kTraceThreads, std::max(1, per_sm) * c->n_sm);
@@ -1355,10 +1389,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
       p.chunks = dptr<Chunk>(c->chunks) + first[b];
       p.n_chunks = first[b + 1] - first[b];
       p.chunk_cursor = dptr<uint32_t>(c->cursor) + b;
-      if (s.info.skip_empty)
-        FFB_TRY((launch_fused<true>(c, p, false, st)));
-      else
-        FFB_TRY((launch_fused<false>(c, p, false, st)));
+      FFB_TRY(launch_fused(c, p, false, st));
     }
     if (packed && bounds[b + 1] > bounds[b]) {
       const int rows = bounds[b + 1] - bounds[b];
@@ -1505,9 +1536,7 @@ int ffb_trace_slice(ffb_ctx* c, long long first, long long count, void* stream)
   // slices of one prepared trace run in stream order, so one cursor serves them all
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   FFB_CUDA(cudaMemsetAsync(p.chunk_cursor, 0, sizeof(uint32_t), st));
-  if (c->main.info.skip_empty)
-    return launch_fused<true>(c, p, false, st);
-  return launch_fused<false>(c, p, false, st);
+  return launch_fused(c, p, false, st);
 }
 
 int ffb_trace_span(ffb_ctx* c, unsigned long long* start_ns, unsigned long long* end_ns)
@@ -1655,10 +1684,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
     p.scene.face_to_row = dptr<int32_t>(c->rows);
     p.scene.face_base = 0;
     p.scene.n_cols = n_meshes;
-    if (s.info.skip_empty)
-      FFB_TRY((launch_fused<true>(c, p, true)));
-    else
-      FFB_TRY((launch_fused<false>(c, p, true)));
+    FFB_TRY(launch_fused(c, p, true));
   }
   std::vector<long long> sums((size_t)n_meshes);
   FFB_CUDA(cudaMemcpyAsync(sums.data(), c->absorb.ptr, sizeof(long long) * sums.size(), cudaMemcpyDeviceToHost,
@@ -1734,8 +1760,7 @@ extern "C" int ffb_parallel_rays(ffb_ctx* c, const ffb_disc_source* src, long lo
   if (n_rays) {
     const GridView g = make_view(s);
     const bool stats = c->stats_on;
-    auto kern = s.info.skip_empty ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<true, false>)
-                                  : (stats ? k_parallel_rays<false, true> : k_parallel_rays<false, false>);
+    auto kern = stats ? k_parallel_rays<true> : k_parallel_rays<false>;
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const long long wave = (long long)std::max(per_sm, 1) * c->n_sm;
@@ -2491,10 +2516,7 @@ extern "C" int ffb_batch_launch(ffb_ctx* c, uint32_t* counts, const unsigned lon
     slot.n_cols = c->batch[s].n_faces;
     cudaStream_t st = c->batch_streams[k++ % kSide];
     const int shape = s < (int)c->batch_shape.size() ? c->batch_shape[(size_t)s] : 0;
-    if (c->batch[s].info.skip_empty)
-      FFB_TRY((launch_fused<true>(c, p, false, st, shape)));
-    else
-      FFB_TRY((launch_fused<false>(c, p, false, st, shape)));
+    FFB_TRY(launch_fused(c, p, false, st, shape));
   }
   for (int j = 0; j < kSide; ++j) {
     FFB_CUDA(cudaEventRecord(c->batch_join[j], c->batch_streams[j]));

@@ -196,11 +196,7 @@ constexpr int kRefillMin = FFB_REFILL_MIN;
 // the order of their directions (bins of an 8 x 8 Morton order on the Malley
 // disk) instead of in index order, so that lanes refilled together trace
 // rays of similar direction from the same face.
-// With `lanes` = K > 0, each lane keeps K rays in shared memory instead of
-// one in registers, and each iteration the warp runs ONE body -- the cell
-// advances or the triangle tests -- chosen by a vote of its lanes, each lane
-// working on one of its rays in that phase; `refill` is then the number of
-// lanes with a free ray slot that triggers a refill.
+// `lanes` (rays per lane kept in shared memory) is 0 in every shape.
 struct TraceShape {
   int adv, test, refill, blocks, coherent, lanes;
 };
@@ -215,11 +211,11 @@ __host__ __device__ constexpr TraceShape trace_shape(int v)
        : v == 6 ? TraceShape{2, 2, 6, 6, 0, 0}
        : v == 7 ? TraceShape{2, 2, 6, 8, 1, 0}
        : v == 8 ? TraceShape{2, 2, 10, 8, 1, 0}
-       : v == 9 ? TraceShape{2, 2, 8, 8, 0, 2}
-       : v == 10 ? TraceShape{2, 2, 8, 8, 1, 2}
-       : v == 11 ? TraceShape{2, 2, 8, 8, 0, 3}
-       : v == 12 ? TraceShape{2, 3, 8, 8, 0, 2}
-       : v == 13 ? TraceShape{2, 3, 8, 8, 0, 3}
+       : v == 9 ? TraceShape{2, 2, 8, 7, 0, 0}
+       : v == 10 ? TraceShape{2, 4, 8, 8, 0, 0}
+       : v == 11 ? TraceShape{4, 2, 8, 8, 0, 0}
+       : v == 12 ? TraceShape{2, 3, 8, 8, 0, 0}
+       : v == 13 ? TraceShape{3, 2, 8, 8, 1, 0}
                  : TraceShape{FFB_ADV_PER_ITER, FFB_TEST_PER_ITER, FFB_REFILL_MIN, FFB_MIN_BLOCKS, 0, 0};
 }
 
@@ -284,73 +280,7 @@ __device__ __forceinline__ void direction_order(uint32_t face, uint32_t j0, int 
   __syncwarp();
 }
 
-// Ray state of the shared-memory lanes (TraceShape::lanes): field f of the
-// ray in column c at R[f * kCols + c], 32-bit words, kCols = K * 128.  The cell
-// coordinates (each below 256) and the empty-space distance (below 128) share
-// one word; the direction signs are recomputed from the direction.
-enum {
-  kRayOx, kRayOy, kRayOz, kRayDx, kRayDy, kRayDz, kRayIx, kRayIy, kRayIz, kRayDlen, kRayBest, kRayBestRef, kRayI,
-  kRayEn, kRayCell, kRayRow, kRayFields
-};
-template <int kCols>
-__device__ __forceinline__ void lane_ray_load(const uint32_t* R, int c, Tracer& T)
-{
-  T.o = f3(__uint_as_float(R[kRayOx * kCols + c]), __uint_as_float(R[kRayOy * kCols + c]),
-           __uint_as_float(R[kRayOz * kCols + c]));
-  T.dir = f3(__uint_as_float(R[kRayDx * kCols + c]), __uint_as_float(R[kRayDy * kCols + c]),
-             __uint_as_float(R[kRayDz * kCols + c]));
-  T.inv = f3(__uint_as_float(R[kRayIx * kCols + c]), __uint_as_float(R[kRayIy * kCols + c]),
-             __uint_as_float(R[kRayIz * kCols + c]));
-  T.dlen = __uint_as_float(R[kRayDlen * kCols + c]);
-  T.best = __uint_as_float(R[kRayBest * kCols + c]);
-  T.best_ref = (int)R[kRayBestRef * kCols + c];
-  T.i = R[kRayI * kCols + c];
-  T.en = R[kRayEn * kCols + c];
-  const uint32_t cell = R[kRayCell * kCols + c];
-  T.cx = (int)(cell & 0xFFu);
-  T.cy = (int)((cell >> 8) & 0xFFu);
-  T.cz = (int)((cell >> 16) & 0xFFu);
-  T.jump = (int)(cell >> 24);
-  T.sx = sgn(T.dir.x);
-  T.sy = sgn(T.dir.y);
-  T.sz = sgn(T.dir.z);
-}
-
-template <int kCols>
-__device__ __forceinline__ void lane_ray_store_cell(uint32_t* R, int c, const Tracer& T)
-{
-  R[kRayI * kCols + c] = T.i;
-  R[kRayEn * kCols + c] = T.en;
-  R[kRayCell * kCols + c] =
-      (uint32_t)T.cx | ((uint32_t)T.cy << 8) | ((uint32_t)T.cz << 16) | ((uint32_t)T.jump << 24);
-}
-
-template <int kCols>
-__device__ __forceinline__ void lane_ray_store_test(uint32_t* R, int c, const Tracer& T)
-{
-  R[kRayBest * kCols + c] = __float_as_uint(T.best);
-  R[kRayBestRef * kCols + c] = (uint32_t)T.best_ref;
-  R[kRayI * kCols + c] = T.i;
-}
-
-template <int kCols>
-__device__ __forceinline__ void lane_ray_store(uint32_t* R, int c, const Tracer& T)
-{
-  R[kRayOx * kCols + c] = __float_as_uint(T.o.x);
-  R[kRayOy * kCols + c] = __float_as_uint(T.o.y);
-  R[kRayOz * kCols + c] = __float_as_uint(T.o.z);
-  R[kRayDx * kCols + c] = __float_as_uint(T.dir.x);
-  R[kRayDy * kCols + c] = __float_as_uint(T.dir.y);
-  R[kRayDz * kCols + c] = __float_as_uint(T.dir.z);
-  R[kRayIx * kCols + c] = __float_as_uint(T.inv.x);
-  R[kRayIy * kCols + c] = __float_as_uint(T.inv.y);
-  R[kRayIz * kCols + c] = __float_as_uint(T.inv.z);
-  R[kRayDlen * kCols + c] = __float_as_uint(T.dlen);
-  lane_ray_store_test<kCols>(R, c, T);
-  lane_ray_store_cell<kCols>(R, c, T);
-}
-
-template <bool kSkip, bool kStats, bool kHash, bool kPower = false, int kShape = 0>
+template <bool kStats, bool kHash, bool kPower = false, int kShape = 0>
 __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     k_form_factors(const __grid_constant__ TraceParams p)
 {
@@ -359,8 +289,8 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
   // coherent hand-out: per warp, direction-bin counters and the chunk's ray order
   __shared__ uint32_t s_bins[kS.coherent ? kWarpsPerBlock * kDirBins : 1];
   __shared__ uint8_t s_perm[kS.coherent ? kWarpsPerBlock * kChunkRaysMax : 1];
-  // K rays per lane: kRayFields fields of kTraceThreads * K slots
-  __shared__ uint32_t s_rays[kS.lanes ? kRayFields * kTraceThreads * kS.lanes : 1];
+  // each lane's ray for the exact test: (origin, direction x), (direction y, z, start distance, row)
+  __shared__ float4 s_ray[2][kTraceThreads];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (p.span && threadIdx.x == 0)
     atomicMin(p.span, global_ns());
@@ -387,145 +317,9 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
   }
   bool exhausted = false;
   uint32_t n_tests = 0, n_cells = 0, n_rays = 0, n_hits = 0, n_jumps = 0;
-  if constexpr (kS.lanes > 0) {
-    // ---- K rays per lane in shared memory, one body per iteration ----
-    constexpr int K = kS.lanes;
-    constexpr int kCols = K * kTraceThreads;
-    uint32_t* const R = s_rays;
-    // the fields of slot k of this lane: column (warp * K + k) * 32 + lane,
-    // so that the 32 lanes of a warp always hit 32 different banks
-    const int col0 = warp * K * 32 + lane;
-    uint32_t ph = 0;  // 2 bits per slot: 0 free, 1 cell exhausted (advance), 2 references pending (test)
-    for (;;) {
-      bool has_free = false, has_adv = false, has_test = false;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const uint32_t s = (ph >> (2 * k)) & 3u;
-        has_free |= s == 0u;
-        has_adv |= s == 1u;
-        has_test |= s == 2u;
-      }
-      unsigned need = __ballot_sync(kFull, has_free);
-      const unsigned busy = __ballot_sync(kFull, has_adv || has_test);
-      if (__popc(need) < kS.refill && busy)
-        need = 0;
-      while (need && !exhausted) {
-        if (c_left == 0) {
-          int k = 0;
-          if (lane == 0)
-            k = (int)atomicAdd(p.chunk_cursor, 1u);
-          k = __shfl_sync(kFull, k, 0);
-          if (k >= p.n_chunks) {
-            exhausted = true;
-            break;
-          }
-          const Chunk ch = p.chunks[k];
-          c_face = ch.face;
-          c_j = ch.j0;
-          c_left = ch.count;
-          c_front = ch.front;
-          c_row = S.face_to_row ? __ldg(S.face_to_row + ch.face) : ch.face;
-          c_pos = 0;
-          if (kS.coherent)
-            direction_order((uint32_t)c_face, (uint32_t)c_j, c_left, key0, key1, epoch, s_bins + warp * kDirBins,
-                            s_perm + warp * kChunkRaysMax, lane);
-        }
-        const int take = min(__popc(need), c_left);
-        const int rank = __popc(need & lane_below);
-        const bool mine = ((need >> lane) & 1u) && rank < take;
-        if (mine) {
-          const int j = c_j + (kS.coherent ? (int)s_perm[warp * kChunkRaysMax + c_pos + rank] : c_pos + rank);
-          float3 o, e;
-          emit_ray(p.frames + 20 * ((size_t)S.face_base + c_face), (uint32_t)c_face, (uint32_t)j, c_front, key0,
-                   key1, epoch, o, e);
-          ++n_rays;
-          Tracer T;
-          if (tracer_begin<kSkip>(T, S.g, o, e, n_cells)) {
-            int k = 0;
-            while (k < K - 1 && ((ph >> (2 * k)) & 3u) != 0u)
-              ++k;
-            const int c = col0 + 32 * k;
-            lane_ray_store<kCols>(R, c, T);
-            R[kRayRow * kCols + c] = (uint32_t)(kPower ? 2 * c_face + (j >= c_front ? 1 : 0) : c_row);
-            ph |= (T.i < T.en ? 2u : 1u) << (2 * k);
-          }
-        }
-        need &= ~__ballot_sync(kFull, mine);
-        c_pos += take;
-        c_left -= take;
-      }
-      has_adv = has_test = false;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const uint32_t s = (ph >> (2 * k)) & 3u;
-        has_adv |= s == 1u;
-        has_test |= s == 2u;
-      }
-      const unsigned va = __ballot_sync(kFull, has_adv), vt = __ballot_sync(kFull, has_test);
-      if (exhausted && !(va | vt))
-        break;
-      const bool do_test = __popc(vt) >= __popc(va);
-      int hit = -1, row = 0;
-      if (do_test ? has_test : has_adv) {
-        const uint32_t want = do_test ? 2u : 1u;
-        int k = 0;
-        while (k < K - 1 && ((ph >> (2 * k)) & 3u) != want)
-          ++k;
-        const int c = col0 + 32 * k;
-        Tracer T;
-        lane_ray_load<kCols>(R, c, T);
-        uint32_t s;
-        if (do_test) {
-#pragma unroll
-          for (int t = 0; t < kS.test; ++t)
-            if (T.i < T.en)
-              tracer_test(T, S.g, n_tests);
-          lane_ray_store_test<kCols>(R, c, T);
-          s = T.i < T.en ? 2u : 1u;
-        } else {
-          bool live = true;
-#pragma unroll
-          for (int a = 0; a < kS.adv; ++a)
-            if (live && T.i >= T.en)
-              live = tracer_advance<kSkip>(T, S.g, n_cells, n_jumps);
-          if (!live) {
-            hit = tracer_result(T, S.g);
-            row = (int)R[kRayRow * kCols + c];
-            s = 0u;
-          } else {
-            lane_ray_store_cell<kCols>(R, c, T);
-            s = T.i < T.en ? 2u : 1u;
-          }
-        }
-        ph = (ph & ~(3u << (2 * k))) | (s << (2 * k));
-      }
-      bool fresh = false;
-      if (hit >= 0) {
-        ++n_hits;
-        const int hcol = S.face_to_row ? __ldg(S.face_to_row + hit) : hit;
-        if (kPower) {
-          atomicAdd(p.absorb + hcol, __ldg(p.power + row));
-        } else {
-          const uint32_t key = (uint32_t)row * (uint32_t)S.n_cols + (uint32_t)hcol;
-          if (kHash)
-            fresh = warp_hash_add(keys, vals, key, S.counts);
-          else
-            atomicAdd(S.counts + key, 1u);
-        }
-      }
-      if (kHash) {
-        fill += __popc(__ballot_sync(kFull, fresh));
-        if (fill > kWarpHash / 2) {
-          warp_hash_flush(keys, vals, S.counts, lane);
-          fill = 0;
-        }
-      }
-    }
-  } else {
   // lane state
   Tracer T;
   bool active = false;
-  int my_row = 0;
   for (;;) {
     unsigned need = __ballot_sync(kFull, !active);
 
@@ -561,8 +355,12 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
         emit_ray(p.frames + 20 * ((size_t)S.face_base + c_face), (uint32_t)c_face, (uint32_t)j, c_front, key0, key1,
                  epoch, o, e);
         ++n_rays;
-        my_row = kPower ? 2 * c_face + (j >= c_front ? 1 : 0) : c_row;
-        active = tracer_begin<kSkip>(T, S.g, o, e, n_cells);
+        const float3 dir = sub3(e, o);
+        float t0;
+        active = tracer_begin<false>(T, S.g, o, dir, &t0, n_cells);
+        s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
+        s_ray[1][threadIdx.x] =
+            make_float4(dir.y, dir.z, t0, __int_as_float(kPower ? 2 * c_face + (j >= c_front ? 1 : 0) : c_row));
       }
       need &= ~__ballot_sync(kFull, mine);
       c_pos += take;
@@ -570,27 +368,32 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     }
     if (exhausted && !__any_sync(kFull, active))
       break;
-    int hit = -1;
+    int hit = -1, open = -1;
     if (active) {
       bool live = true;
 #pragma unroll
       for (int k = 0; k < kS.adv; ++k)
         if (live && T.i >= T.en)
-          live = tracer_advance<kSkip>(T, S.g, n_cells, n_jumps);
+          live = tracer_advance(T, S.g, n_cells, n_jumps);
       if (!live) {
         active = false;
-        hit = tracer_result(T, S.g);
+        hit = T.face;
       } else {
 #pragma unroll
         for (int k = 0; k < kS.test; ++k)
-          if (T.i < T.en)
-            tracer_test(T, S.g, n_tests);
+          if (T.i < T.en && open < 0)
+            open = tracer_test<false>(T, S.g, n_tests);
       }
+    }
+    if (open >= 0) {
+      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
+      tracer_exact(T, S.g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
     }
     bool fresh = false;
     if (hit >= 0) {
       ++n_hits;
       const int col = S.face_to_row ? __ldg(S.face_to_row + hit) : hit;
+      const int my_row = __float_as_int(s_ray[1][threadIdx.x].w);
       if (kPower) {
         atomicAdd(p.absorb + col, __ldg(p.power + my_row));
       } else {
@@ -609,7 +412,6 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
       }
     }
   }
-  }  // one ray per lane in registers
   if (kHash)
     warp_hash_flush(keys, vals, S.counts, lane);
   if (kStats)
@@ -628,13 +430,14 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
 // reference chooses the front absorbance) and to side_counts[2h + 1]
 // otherwise.
 // ---------------------------------------------------------------------------
-template <bool kSkip, bool kStats>
+template <bool kStats>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_parallel_rays(GridView g, const __grid_constant__ DiscSource src, const float* __restrict__ faces9,
                     unsigned long long n_rays, uint32_t key0, uint32_t key1, uint32_t epoch,
                     uint32_t* __restrict__ side_counts, unsigned long long* __restrict__ cursor,
                     unsigned long long* __restrict__ stats)
 {
+  __shared__ float4 s_ray[2][kTraceThreads];  // as in k_form_factors
   const int lane = threadIdx.x & 31;
   const unsigned lane_below = (1u << lane) - 1u;
   uint32_t n_tests = 0, n_cells = 0, n_done = 0, n_hits = 0, n_jumps = 0;
@@ -656,21 +459,26 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           float3 o, e;
           emit_disc_ray(src, j, key0, key1, epoch, o, e);
           ++n_done;
-          active = tracer_begin<kSkip>(T, g, o, e, n_cells);
+          const float3 dir = sub3(e, o);
+          float t0;
+          active = tracer_begin<true>(T, g, o, dir, &t0, n_cells);
+          s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
+          s_ray[1][threadIdx.x] = make_float4(dir.y, dir.z, t0, 0.f);
         }
       }
     }
     if (exhausted && !__any_sync(kFull, active))
       break;
+    int open = -1;
     if (active) {
       bool live = true;
 #pragma unroll
       for (int k = 0; k < FFB_ADV_PER_ITER; ++k)
         if (live && T.i >= T.en)
-          live = tracer_advance<kSkip>(T, g, n_cells, n_jumps);
+          live = tracer_advance(T, g, n_cells, n_jumps);
       if (!live) {
         active = false;
-        const int h = tracer_result(T, g);
+        const int h = T.face;
         if (h >= 0) {
           ++n_hits;
           // triangle_normal (math/triangle.cpp:114-119), dot with the direction
@@ -684,9 +492,13 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
       } else {
 #pragma unroll
         for (int k = 0; k < FFB_TEST_PER_ITER; ++k)
-          if (T.i < T.en)
-            tracer_test(T, g, n_tests);
+          if (T.i < T.en && open < 0)
+            open = tracer_test<true>(T, g, n_tests);
       }
+    }
+    if (open >= 0) {
+      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
+      tracer_exact(T, g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
     }
   }
   if (kStats)
@@ -721,12 +533,12 @@ __global__ void k_epoch_bump(uint32_t* epoch)
 // hit_point (optional) gets the point, NaN for a miss.  Persistent warps take
 // rays from a global cursor (one atomic per refill) as lanes fall idle.
 // ---------------------------------------------------------------------------
-template <bool kSkip>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_cast(GridView g, const float* __restrict__ rays6, long n_rays, int32_t* __restrict__ hit_face,
            float* __restrict__ hit_point, unsigned long long* __restrict__ stats,
            unsigned long long* __restrict__ cursor)
 {
+  __shared__ float4 s_ray[2][kTraceThreads];  // as in k_form_factors
   const int lane = threadIdx.x & 31;
   const unsigned lane_below = (1u << lane) - 1u;
   uint32_t n_tests = 0, n_cells = 0, n_done = 0, n_hits = 0, n_jumps = 0;
@@ -762,7 +574,11 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           const float* q = rays6 + 6 * r;
           const float3 o = f3(__ldg(q + 0), __ldg(q + 1), __ldg(q + 2));
           const float3 e = f3(__ldg(q + 3), __ldg(q + 4), __ldg(q + 5));
-          active = tracer_begin<kSkip>(T, g, o, e, n_cells);
+          const float3 dir = sub3(e, o);
+          float t0;
+          active = tracer_begin<true>(T, g, o, dir, &t0, n_cells);
+          s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
+          s_ray[1][threadIdx.x] = make_float4(dir.y, dir.z, t0, 0.f);
           if (!active)
             finish(id, -1, o);
         }
@@ -770,21 +586,31 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     }
     if (exhausted && !__any_sync(kFull, active))
       break;
+    int open = -1;
     if (active) {
       bool live = true;
 #pragma unroll
       for (int k = 0; k < FFB_ADV_PER_ITER; ++k)
         if (live && T.i >= T.en)
-          live = tracer_advance<kSkip>(T, g, n_cells, n_jumps);
+          live = tracer_advance(T, g, n_cells, n_jumps);
       if (!live) {
         active = false;
-        finish(id, tracer_result(T, g), T.best_pt);
+        float3 pt = f3(0.f, 0.f, 0.f);
+        if (hit_point && T.face >= 0) {  // the reference's hit point
+          const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
+          tri_hit(reinterpret_cast<const float4*>(g.tri + T.face), f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), pt);
+        }
+        finish(id, T.face, pt);
       } else {
 #pragma unroll
         for (int k = 0; k < FFB_TEST_PER_ITER; ++k)
-          if (T.i < T.en)
-            tracer_test(T, g, n_tests);
+          if (T.i < T.en && open < 0)
+            open = tracer_test<true>(T, g, n_tests);
       }
+    }
+    if (open >= 0) {
+      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
+      tracer_exact(T, g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
     }
   }
   warp_stats(stats, n_tests, n_cells, n_done, n_hits, n_jumps);
