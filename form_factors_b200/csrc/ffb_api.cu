@@ -68,7 +68,8 @@ struct DevBuf {
   size_t cap = 0;
 };
 
-constexpr int kChunkRays = 256;  // rays per work chunk of the fused kernel
+constexpr int kChunkRays = 256;  // rays per work chunk of the fused kernel at most
+constexpr int kTailRays = 64;    // rays per chunk of a launch's last sixteenth at most
 static_assert(kChunkRays == kChunkRaysMax, "the coherent hand-out orders whole chunks");
 constexpr int kMaxRows = 65535;  // matrix index row * n + col stays below 0xFFFFFFFF
 constexpr int kMaxPipeBlocks = 16;  // row blocks of a pipelined host output
@@ -602,18 +603,35 @@ int grid_build(ffb_ctx* c, SceneData& s, const ffb_grid_params* params)
   return FFB_OK;
 }
 
+// Rays per chunk of a launch of `total` rays.  A small launch spreads over the
+// GPU instead of running 256 rays after one another in a few warps: at least
+// four chunks per warp where that many rays are left (24 000 rays of 12 faces:
+// 96 warps and 171 us with 256-ray chunks, 750 warps and 27 us with 32).
+// Larger launches keep 256 rays: each chunk costs its warp an atomic on the
+// shared cursor and breaks a refill (64-ray chunks on 3.5 M-ray scenes: 4 %
+// slower).
+int chunk_rays(const ffb_ctx* c, long long total)
+{
+  const long long warps = 32ll * c->n_sm;
+  int rays = kChunkRays;
+  while (rays > 32 && total < rays * warps * 4)
+    rays /= 2;
+  return rays;
+}
+
 // Chunk table of the emitting faces `faces` (in launch order) built on the
 // device: the host computes each face's first chunk (work linear in faces,
 // not in rays) and uploads 16 bytes per face; k_chunk_fill writes the
-// chunks.  first[i] gets the first chunk of faces[i], *n_chunks the total.
-int device_chunks(ffb_ctx* c, const std::vector<int32_t>& faces, const int32_t* front, const int32_t* rear,
+// chunks, of `size` rays.  first[i] gets the first chunk of faces[i],
+// *n_chunks the total.
+int device_chunks(ffb_ctx* c, const std::vector<int32_t>& faces, const int32_t* front, const int32_t* rear, int size,
                   std::vector<long long>& first, long long* n_chunks, bool short_tail = false)
 {
   // With short_tail, the faces that hold the last sixteenth of the rays get
   // chunks of kTailRays: the launch's last chunks are short, so its warps
   // run out of work closer together (a 256-ray chunk takes a warp about as
   // long as 1/18 of a full-GPU launch).
-  constexpr int kTailRays = 64;
+  const int tail_size = std::min(size, kTailRays);
   long long tail_from = LLONG_MAX;
   if (short_tail) {
     long long all = 0;
@@ -630,10 +648,11 @@ int device_chunks(ffb_ctx* c, const std::vector<int32_t>& faces, const int32_t* 
     const long long nf = (long long)front[f] + rear[f];
     if (nf > INT_MAX - kChunkRays)
       return fail(FFB_ERR_TOO_LARGE, "face %d emits %lld rays; at most %d", f, nf, INT_MAX - kChunkRays);
-    const int size = rays >= tail_from ? kTailRays : kChunkRays;
+    const bool is_tail = rays >= tail_from;
+    const int per = is_tail ? tail_size : size;
     first[i] = next;
-    (size == kChunkRays ? head : tail).push_back(make_int4(f, front[f], (int)nf, (int)next));
-    next += (nf + size - 1) / size;
+    (is_tail ? tail : head).push_back(make_int4(f, front[f], (int)nf, (int)next));
+    next += (nf + per - 1) / per;
     rays += nf;
     if (next > INT_MAX)
       return fail(FFB_ERR_TOO_LARGE, "more than %d work chunks", INT_MAX);
@@ -646,11 +665,11 @@ int device_chunks(ffb_ctx* c, const std::vector<int32_t>& faces, const int32_t* 
     head.insert(head.end(), tail.begin(), tail.end());
     FFB_TRY(upload(c, c->chunk_src, head.data(), sizeof(int4) * head.size()));
     if (nh)
-      k_chunk_fill<kChunkRays><<<grid_blocks((long long)nh * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-          dptr<int4>(c->chunk_src), (int)nh, dptr<Chunk>(c->chunks));
+      k_chunk_fill<<<grid_blocks((long long)nh * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
+          dptr<int4>(c->chunk_src), (int)nh, size, dptr<Chunk>(c->chunks));
     if (!tail.empty())
-      k_chunk_fill<kTailRays><<<grid_blocks((long long)tail.size() * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-          dptr<int4>(c->chunk_src) + nh, (int)tail.size(), dptr<Chunk>(c->chunks));
+      k_chunk_fill<<<grid_blocks((long long)tail.size() * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
+          dptr<int4>(c->chunk_src) + nh, (int)tail.size(), tail_size, dptr<Chunk>(c->chunks));
     FFB_CUDA(cudaGetLastError());
   }
   return FFB_OK;
@@ -1268,9 +1287,12 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   }
   // emitting faces block after block (ascending within a block)
   std::vector<std::vector<int32_t>> by_block(n_blocks);
+  long long emitted = 0;  // rays of the row range
   for (int f = 0; f < s.n_faces; ++f)
-    if (face_block[f] >= 0 && front[f] + (long long)rear[f] > 0)
+    if (face_block[f] >= 0 && front[f] + (long long)rear[f] > 0) {
       by_block[face_block[f]].push_back(f);
+      emitted += front[f] + (long long)rear[f];
+    }
   std::vector<int32_t> order;
   order.reserve((size_t)s.n_faces);
   std::vector<size_t> block_pos(n_blocks + 1, 0);
@@ -1281,7 +1303,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   block_pos[n_blocks] = order.size();
   std::vector<long long> face_first;
   long long n_chunks = 0;
-  FFB_TRY(device_chunks(c, order, front, rear, face_first, &n_chunks, n_blocks == 1));
+  FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, emitted / n_blocks), face_first, &n_chunks, n_blocks == 1));
   std::vector<int> first(n_blocks + 1, 0);
   for (int b = 0; b <= n_blocks; ++b)
     first[b] = (int)(block_pos[b] < order.size() ? face_first[block_pos[b]] : n_chunks);
@@ -1491,7 +1513,7 @@ int ffb_trace_prepare(ffb_ctx* c, const int32_t* front, const int32_t* rear, uin
       order.push_back(f);
   std::vector<long long> first;
   long long nch = 0;
-  FFB_TRY(device_chunks(c, order, front, rear, first, &nch));
+  FFB_TRY(device_chunks(c, order, front, rear, kChunkRays, first, &nch));
   FFB_TRY(ensure(c, c->cursor, sizeof(uint32_t) * kMaxPipeBlocks));
   FFB_TRY(ensure(c, c->span, 2 * sizeof(unsigned long long)));
   const unsigned long long span0[2] = {~0ull, 0ull};
@@ -1655,7 +1677,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
       order.push_back(f);
   std::vector<long long> face_first;
   long long n_chunks = 0;
-  FFB_TRY(device_chunks(c, order, front, rear, face_first, &n_chunks, true));
+  FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, total), face_first, &n_chunks, true));
   FFB_TRY(ensure(c, c->absorb, sizeof(unsigned long long) * (size_t)n_meshes));
   FFB_CUDA(cudaMemsetAsync(c->absorb.ptr, 0, sizeof(unsigned long long) * (size_t)n_meshes, c->stream));
   FFB_TRY(ensure(c, c->stats, sizeof(unsigned long long) * kStatSlots));
@@ -2387,7 +2409,7 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
   // first chunk): the host's work and upload are linear in faces, not rays.
   // As in a single-scene launch, the faces holding the last sixteenth of a
   // scene's rays get 64-ray chunks (its launch's tail is shorter).
-  constexpr int kTailRays = 64;
+  const int chunk = chunk_rays(c, total), tail_chunk = std::min(chunk, kTailRays);
   std::vector<int4> src, tail;
   src.reserve((size_t)n_all);
   c->batch_chunk_first.assign(n_scenes + 1, 0);
@@ -2406,9 +2428,10 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
       if (nf > INT_MAX - kChunkRays)
         return fail(FFB_ERR_TOO_LARGE, "scene %d face %d emits %lld rays; at most %d", s, f, nf,
                     INT_MAX - kChunkRays);
-      const int size = rays >= tail_from ? kTailRays : kChunkRays;
-      (size == kChunkRays ? src : tail).push_back(make_int4(f, front[f0 + f], (int)nf, (int)next));
-      next += (nf + size - 1) / size;
+      const bool is_tail = rays >= tail_from;
+      const int per = is_tail ? tail_chunk : chunk;
+      (is_tail ? tail : src).push_back(make_int4(f, front[f0 + f], (int)nf, (int)next));
+      next += (nf + per - 1) / per;
       rays += nf;
       if (next > INT_MAX)
         return fail(FFB_ERR_TOO_LARGE, "more than %d work chunks", INT_MAX);
@@ -2422,11 +2445,11 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
     src.insert(src.end(), tail.begin(), tail.end());  // one staged upload
     FFB_TRY(upload(c, c->chunk_src, src.data(), sizeof(int4) * src.size()));
     if (nh)
-      k_chunk_fill<kChunkRays><<<grid_blocks((long long)nh * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-          dptr<int4>(c->chunk_src), (int)nh, dptr<Chunk>(c->batch_chunks));
+      k_chunk_fill<<<grid_blocks((long long)nh * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
+          dptr<int4>(c->chunk_src), (int)nh, chunk, dptr<Chunk>(c->batch_chunks));
     if (!tail.empty())
-      k_chunk_fill<kTailRays><<<grid_blocks((long long)tail.size() * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
-          dptr<int4>(c->chunk_src) + nh, (int)tail.size(), dptr<Chunk>(c->batch_chunks));
+      k_chunk_fill<<<grid_blocks((long long)tail.size() * 32, 256, c->n_sm * 8), 256, 0, c->stream>>>(
+          dptr<int4>(c->chunk_src) + nh, (int)tail.size(), tail_chunk, dptr<Chunk>(c->batch_chunks));
     FFB_CUDA(cudaGetLastError());
   }
   std::vector<uint2> keys((size_t)n_scenes);

@@ -19,17 +19,16 @@ struct Chunk {
 
 // Writes the work chunks of the emitting faces: src[i] = {face, front rays,
 // front + rear rays, first chunk}; the face's rays [0, nf) become chunks of
-// kRays consecutive rays (the last one shorter), one warp per face.
-template <int kRays>
-__global__ void k_chunk_fill(const int4* __restrict__ src, int n, Chunk* __restrict__ chunks)
+// `rays` consecutive rays (the last one shorter), one warp per face.
+__global__ void k_chunk_fill(const int4* __restrict__ src, int n, int rays, Chunk* __restrict__ chunks)
 {
   const int lane = threadIdx.x & 31;
   const int warps = (int)((gridDim.x * blockDim.x) >> 5);
   for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < n; i += warps) {
     const int4 f = src[i];
-    const int nc = (f.z + kRays - 1) / kRays;
+    const int nc = (f.z + rays - 1) / rays;
     for (int j = lane; j < nc; j += 32)
-      chunks[(uint32_t)f.w + (uint32_t)j] = Chunk{f.x, j * kRays, min(kRays, f.z - j * kRays), f.y};
+      chunks[(uint32_t)f.w + (uint32_t)j] = Chunk{f.x, j * rays, min(rays, f.z - j * rays), f.y};
   }
 }
 
