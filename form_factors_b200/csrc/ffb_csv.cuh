@@ -200,17 +200,6 @@ __host__ __device__ inline Dec6 round6_general(uint32_t m, int q)
   return round6_from_7(n7, !big_zero(a), exp10);
 }
 
-// Text sinks of the formatter: a pointer (host buffers, shared memory) or a
-// counter (lengths only; the compiler drops the character work).
-struct PtrOut {
-  char* p;
-  int n;
-  __host__ __device__ void put(char c) { p[n++] = c; }
-};
-struct CountOut {
-  int n;
-  __host__ __device__ void put(char) { ++n; }
-};
 
 template <class Out>
 __host__ __device__ inline void put_text(Out& out, const char* t)
@@ -297,19 +286,127 @@ __host__ __device__ inline void format_g6_to(float f, Out& out)
     out.put(next_digit());
 }
 
+// An entry's text in registers: its first 16 bytes, little endian, and the
+// length.  The longest entry has 12 characters.
+struct Text {
+  uint64_t lo, hi;
+  int len;
+
+  __host__ __device__ void put(char c)
+  {
+    if (len < 8)
+      lo |= (uint64_t)(uint8_t)c << (8 * len);
+    else
+      hi |= (uint64_t)(uint8_t)c << (8 * (len - 8));
+    ++len;
+  }
+};
+
+__host__ __device__ inline int bit_width64(uint64_t v)
+{
+#ifdef __CUDA_ARCH__
+  return 64 - __clzll((long long)v);
+#else
+  return v ? 64 - __builtin_clzll(v) : 0;
+#endif
+}
+
+// The general formatter's text (a call of its own on the device: it is rare,
+// and its digit arrays would take the other entries' registers).
+#ifdef __CUDACC__
+__noinline__
+#endif
+__host__ __device__ inline Text text_g6_general(float f)
+{
+  Text t{0, 0, 0};
+  format_g6_to(f, t);
+  return t;
+}
+
+// "%g" of f.  Values in [10^-4, 10^6) -- every form factor of a row of up to
+// 10 000 rays -- take a few dozen integer operations: with X the decimal
+// exponent of the value's binade, value * 10^(6 - X) = (m * 5^(6 - X)) >>
+// (s - (6 - X)) is one 64-bit product (m < 2^24, 5^10 < 2^24), whose integer
+// part holds seven or eight digits and whose low bits say whether anything
+// follows them.  The six rounded digits are laid out as bytes and shifted into
+// place.  The rest goes through format_g6_to.
+__host__ __device__ inline Text text_g6(float f)
+{
+  uint32_t bits;
+#ifdef __CUDA_ARCH__
+  bits = __float_as_uint(f);
+#else
+  __builtin_memcpy(&bits, &f, 4);
+#endif
+  const int e2 = (int)((bits >> 23) & 0xFFu) - 127;  // the value's binade [2^e2, 2^(e2 + 1))
+  if (e2 < -13 || e2 > 18)
+    return text_g6_general(f);
+  const uint32_t m = (bits & 0x7FFFFFu) | 0x800000u;
+  int X = (e2 * 315653) >> 20;  // floor(e2 * log10(2)): 10^X <= 2^e2
+  const int k = 6 - X;          // 1 .. 10
+  const uint64_t p5 = (uint64_t)((k & 1 ? 5u : 1u) * (k & 2 ? 25u : 1u) * (k & 4 ? 625u : 1u)) * (k & 8 ? 390625u : 1u);
+  const uint64_t prod = (uint64_t)m * p5;
+  const int sh = 23 - e2 - k;   // at least 3
+  uint32_t n = (uint32_t)(prod >> sh);  // the first 7 digits, or 8
+  bool rest = (prod & ((1ull << sh) - 1ull)) != 0;
+  if (n >= 10000000u) {
+    const uint32_t q = n / 10u;
+    rest |= n != q * 10u;
+    n = q;
+    ++X;
+  }
+  uint32_t v = n / 10u;
+  const uint32_t r = n - v * 10u;
+  v += r > 5u || (r == 5u && (rest || (v & 1u)));
+  if (v == 1000000u) {
+    v = 100000u;
+    ++X;
+  }
+  if (X < -4 || X > 5)
+    return text_g6_general(f);
+  Text t{0, 0, 0};
+  // digits, most significant in the lowest byte
+  const uint32_t h = v / 1000u, l = v - h * 1000u;
+  const uint32_t h1 = h / 100u, h2 = h / 10u, l1 = l / 100u, l2 = l / 10u;
+  const uint64_t digits = (uint64_t)(h1 | (h2 - h1 * 10u) << 8 | (h - h2 * 10u) << 16 | l1 << 24) |
+                          (uint64_t)((l2 - l1 * 10u) | (l - l2 * 10u) << 8) << 32;
+  const int nd = (bit_width64(digits) + 7) >> 3;  // without trailing zeros
+  const uint64_t text = digits + 0x303030303030ull;
+  const uint64_t kept = text & ((1ull << (8 * nd)) - 1ull);
+  if (X >= 0) {
+    const int at = 8 * (X + 1);  // the integer part, zeros included
+    t.len = X + 1;
+    t.lo = text & ((1ull << at) - 1ull);
+    if (nd > X + 1) {
+      t.lo |= (uint64_t)'.' << at | (kept >> at) << (at + 8);
+      t.len = nd + 1;
+    }
+  } else {
+    const int at = 8 * (1 - X);  // "0." and the zeros after the point
+    t.lo = (0x3030302E30ull & ((1ull << at) - 1ull)) | kept << at;
+    t.hi = kept >> (64 - at);
+    t.len = nd + 1 - X;
+  }
+  if (bits >> 31) {
+    t.hi = t.hi << 8 | t.lo >> 56;
+    t.lo = t.lo << 8 | (uint64_t)'-';
+    ++t.len;
+  }
+  return t;
+}
+
 // Writes "%g" of f to out (no terminator); returns the length.
 __host__ __device__ inline int format_g6(float f, char* out)
 {
-  PtrOut o{out, 0};
-  format_g6_to(f, o);
-  return o.n;
+  const Text t = text_g6(f);
+  for (int i = 0; i < t.len; ++i)
+    out[i] = (char)((i < 8 ? t.lo >> (8 * i) : t.hi >> (8 * (i - 8))) & 0xFFu);
+  return t.len;
 }
 
 __host__ __device__ inline int format_g6_len(float f)
 {
-  CountOut o{0};
-  format_g6_to(f, o);
-  return o.n;
+  return text_g6(f).len;
 }
 
 #ifdef __CUDACC__
@@ -436,6 +533,15 @@ __device__ __forceinline__ void enqueue(uint16_t* queue, uint32_t* qn, bool take
   base = __shfl_sync(0xFFFFFFFFu, base, __ffs(mask) - 1);
   if (take)
     queue[base + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)o;
+}
+
+// Stores a text's bytes at any address.
+__device__ __forceinline__ void put_bytes(unsigned char* to, const Text& t)
+{
+#pragma unroll
+  for (int i = 0; i < kMaxEntry - 3; ++i)
+    if (i < t.len)
+      to[i] = (unsigned char)(i < 8 ? t.lo >> (8 * i) : t.hi >> (8 * (i - 8)));
 }
 
 __global__ void __launch_bounds__(kThreads, 4) k_csv_len(Source s, unsigned long long* __restrict__ tile_len)
@@ -599,9 +705,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_csv_write(Source s, const unsig
     const int o = queue[q];
     int col;
     const float v = tile_value(s, tile, o, &col);
-    PtrOut w{reinterpret_cast<char*>(sbuf + off[o]), 0};
-    format_g6_to(v, w);
+    Text w = text_g6(v);
     w.put(col == s.n - 1 ? '\n' : ';');
+    put_bytes(sbuf + off[o], w);
   }
   __syncthreads();
   // 4. copy [shift, shift + total) of sbuf to dst
@@ -621,35 +727,46 @@ __global__ void __launch_bounds__(kThreads, 4) k_csv_write(Source s, const unsig
 // ---------------------------------------------------------------------------
 // Single pass into a device buffer (decoupled look-back).  Each block takes
 // the next tile by ticket, so every tile it waits for already runs and waits
-// only for earlier tiles.  Thread t holds entries [16t, 16t + 16) of its
-// tile, so its text is one contiguous run whose offset comes from a block
-// scan of 16-entry sums; +0 entries ("0" and the separator) are written by
-// their thread, the others formatted densely through the block queue (once
-// for the length, once for the text).  The tile publishes its length and
-// lays its text out in shared memory; then it sums the lengths and prefixes
-// the preceding tiles published (bounded polls), publishes its inclusive
-// prefix and stores its text with 16-byte writes.  A tile whose text would
-// pass the end of the buffer writes nothing and sets kFusedOverflow; the
-// last tile writes the text length.
+// only for earlier tiles.  A warp works through its 512 consecutive entries
+// without block barriers: lane l holds entries 32k + l, ballots give the
+// nonzero ones, which go to the warp's queue in entry order and are formatted
+// by all lanes together; a scan of their lengths gives, for an entry with q
+// nonzeros before it, the offset 2 * entry + extra[q] (a +0 entry is "0" and
+// the separator).  Neighbouring lanes then stage neighbouring bytes.  The tile
+// publishes its length, sums the lengths and prefixes the preceding tiles
+// published (bounded polls), publishes its inclusive prefix and stores its
+// text with 16-byte writes.  A tile whose text would pass the end of the
+// buffer writes nothing and sets kFusedOverflow; the last tile writes the text
+// length.
+//
+// What bounds it: instruction issue (about 50 warp instructions per 32
+// entries); 487 M entries of which 4.5 % are nonzero, 1.06 GB of text: 3.34 ms
+// with a whole tile per barrier phase, each nonzero formatted twice by digit
+// loops and zeros staged by byte stores at a 32-byte stride (eight lanes on a
+// bank); 1.73 ms as it is now.  A warp stages 2 KB of text at a time, which
+// holds its 512 entries unless over a fifth of them are nonzero: shared memory
+// for the longest possible text would leave three blocks per SM.
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kTileAgg = 1ull << 62;     // status: the tile's own length
 constexpr unsigned long long kTilePrefix = 2ull << 62;  // status: the inclusive prefix
 constexpr unsigned long long kTileValue = (1ull << 62) - 1;
 constexpr unsigned kLookbackPolls = 1u << 22;           // polls of one status word before giving up
 enum : unsigned { kFusedTimeout = 1u, kFusedOverflow = 2u };
-constexpr int kRun = 16;  // consecutive entries per thread
-#ifndef FFB_CSV_THREADS
-#define FFB_CSV_THREADS 256
-#endif
-#ifndef FFB_CSV_BLOCKS
-#define FFB_CSV_BLOCKS 3
-#endif
-constexpr int kFusedThreads = FFB_CSV_THREADS;
-constexpr int kFusedTile = kRun * kFusedThreads;              // entries per tile, one run per thread
-constexpr int kFusedText = kFusedTile * (kMaxEntry - 3) + 16;  // staged text of a tile at most, + one word read past it
-static_assert(kFusedText % 16 == 0, "the length bytes start 16-byte aligned");
-constexpr size_t kFusedSmem =
-    kFusedText + kFusedTile * (sizeof(uint8_t) + sizeof(uint16_t)) + kFusedThreads * sizeof(uint32_t);
+constexpr int kFusedThreads = 256;
+constexpr int kFusedWarps = kFusedThreads / 32;
+constexpr int kWarpEntries = 512;
+constexpr int kChunks = kWarpEntries / 32;
+constexpr int kFusedTile = kWarpEntries * kFusedWarps;  // entries per tile
+constexpr int kWindow = 2048;                           // staged text per warp, a multiple of 16
+
+// A warp's shared memory.
+struct WarpText {
+  __align__(16) unsigned char text[kWindow + 16];  // one word is read past the window
+  uint16_t entry[kWarpEntries];                    // nonzero entries, in order
+  uint16_t extra[kWarpEntries + 1];                // sum of (length - 2) of those before
+  uint32_t nonzero[kChunks];                       // their lanes in each chunk of 32
+};
+constexpr size_t kFusedSmem = sizeof(WarpText) * kFusedWarps;
 
 struct FusedSink {
   char* text;
@@ -705,151 +822,257 @@ __device__ __forceinline__ unsigned long long look_back(const FusedSink& out, lo
   }
 }
 
-// Value and column of entry o of a fused tile (queue work, one division).
-__device__ __forceinline__ float fused_value(const Source& s, long long tile, int o, int* col)
+// Entries [e0, e0 + 512) of one warp: where they lie in the matrix.
+struct WarpRows {
+  uint32_t e0;
+  uint32_t row, col;  // of entry e0
+  uint32_t n;
+  int valid;          // entries before the matrix end, at most 512
+
+  // 512 entries of one or two rows, every count of zero a +0 entry
+  bool simple;
+  int row_end;        // simple: the last entry of the first row (past 511 if it goes on)
+  float ratio0, ratio1;  // simple: of the two rows (counts)
+
+  // Separator after entry o, and entry o as text.
+  template <bool kSimple>
+  __device__ __forceinline__ char separator(int o) const
+  {
+    if (kSimple)
+      return o == row_end ? '\n' : ';';
+    uint32_t r, c;
+    locate(o, &r, &c);
+    return c == n - 1 ? '\n' : ';';
+  }
+  template <bool kSimple>
+  __device__ __forceinline__ Text text(const Source& s, const uint32_t* words, int o) const
+  {
+    float v;
+    char sep;
+    if (kSimple) {
+      const uint32_t raw = __ldg(words + o);
+      v = s.ff ? __uint_as_float(raw) : (float)raw * (o > row_end ? ratio1 : ratio0);
+      sep = separator<true>(o);
+    } else {
+      uint32_t r, c;
+      locate(o, &r, &c);
+      v = entry_value(s, (long long)e0 + o, row_ratio(s, (int)r));
+      sep = c == n - 1 ? '\n' : ';';
+    }
+    Text t = text_g6(v);
+    t.put(sep);
+    return t;
+  }
+
+  // row and column of entry o
+  __device__ __forceinline__ void locate(int o, uint32_t* r, uint32_t* c) const
+  {
+    uint32_t k = col + (uint32_t)o;
+    *r = row;
+    if (k >= n) {
+      const uint32_t q = n > (uint32_t)kWarpEntries ? 1u : k / n;
+      *r += q;
+      k -= q * n;
+    }
+    *c = k;
+  }
+};
+
+// Stages the warp's text bytes [w0, w0 + kWindow) at W.text; `first` is the
+// text of the lane's first queue entry.  With kAll the whole text fits the
+// window.
+template <bool kAll, bool kSimple>
+__device__ __forceinline__ void stage_text(const Source& s, const WarpRows& at, const uint32_t* words, WarpText& W, int n_q,
+                                           const Text& first, int w0, int lane)
 {
-  const long long e = tile * kFusedTile + o;
-  const int row = (int)(e / s.n);
-  *col = (int)(e - (long long)row * s.n);
-  return entry_value(s, e, row_ratio(s, row));
+  const uint32_t below = (1u << lane) - 1u;
+  const uint16_t* extra = W.extra;  // of the nonzeros in the chunks before
+#pragma unroll 8
+  for (int k = 0; k < kChunks; ++k) {
+    const uint32_t m = W.nonzero[k];
+    const int o = 32 * k + lane;
+    if (!((m >> lane) & 1u) && (kSimple || o < at.valid)) {
+      const int p = 2 * o + extra[__popc(m & below)] - w0;
+      const unsigned char sep = (unsigned char)at.separator<kSimple>(o);
+      if (kAll || (unsigned)p < (unsigned)kWindow)
+        W.text[p] = '0';
+      if (kAll || (unsigned)(p + 1) < (unsigned)kWindow)
+        W.text[p + 1] = sep;
+    }
+    extra += __popc(m);
+  }
+  for (int q = lane; q < n_q; q += 32) {
+    const int o = W.entry[q];
+    const int p = 2 * o + W.extra[q] - w0;
+    if (!kAll && (p >= kWindow || p + kMaxEntry < 0))
+      continue;
+    Text t = first;
+    if (q >= 32)
+      t = at.text<kSimple>(s, words, o);
+    if (kAll) {
+      put_bytes(W.text + p, t);
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < t.len; ++i)
+        if ((unsigned)(p + i) < (unsigned)kWindow)
+          W.text[p + i] = (unsigned char)(i < 8 ? t.lo >> (8 * i) : t.hi >> (8 * (i - 8)));
+    }
+  }
 }
 
-__global__ void __launch_bounds__(kFusedThreads, FFB_CSV_BLOCKS) k_csv_fused(Source s, FusedSink out)
+// The warp's entries: the nonzero ones queued and formatted (`first` is the
+// text of the lane's first), their lengths scanned.  Returns their number;
+// *len gets the length of the warp's text.
+template <bool kSimple>
+__device__ __forceinline__ int queue_entries(const Source& s, const WarpRows& at, const uint32_t* words,
+                                             const uint32_t (&raw)[kChunks], bool plain, WarpText& W, Text& first,
+                                             int* len, int lane)
+{
+  const uint32_t below = (1u << lane) - 1u;
+  int n_q = 0;
+#pragma unroll
+  for (int k = 0; k < kChunks; ++k) {
+    const int o = 32 * k + lane;
+    bool take = raw[k] != 0u;
+    if (!kSimple && !plain && o < at.valid) {
+      uint32_t r, c;
+      at.locate(o, &r, &c);
+      take = __float_as_uint((float)raw[k] * row_ratio(s, (int)r)) != 0u;
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, take);
+    if (take)
+      W.entry[n_q + __popc(m & below)] = (uint16_t)o;
+    n_q += __popc(m);
+    if (lane == 0)
+      W.nonzero[k] = m;
+  }
+  __syncwarp();
+  int extra = 0;
+  for (int q0 = 0; q0 < n_q; q0 += 32) {
+    const int q = q0 + lane;
+    int mine = 0;
+    if (q < n_q) {
+      const Text t = at.text<kSimple>(s, words, W.entry[q]);
+      mine = t.len - 2;
+      if (q0 == 0)
+        first = t;
+    }
+    int incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= d)
+        incl += y;
+    }
+    if (q < n_q)
+      W.extra[q] = (uint16_t)(extra + incl - mine);
+    extra += __shfl_sync(0xFFFFFFFFu, incl, 31);
+  }
+  if (lane == 0)
+    W.extra[n_q] = (uint16_t)extra;
+  *len = 2 * at.valid + extra;
+  return n_q;
+}
+
+// Copies `len` staged bytes to dst: bytes up to the first 16-byte boundary,
+// then 16-byte stores assembled from 32-bit shared words (funnel shifts by the
+// misalignment), then the tail.
+__device__ __forceinline__ void copy_text(char* dst, const unsigned char* text, uint32_t len, int lane)
+{
+  const uint32_t head = min(len, (uint32_t)((16u - ((uintptr_t)dst & 15u)) & 15u));
+  const uint32_t body = (len - head) >> 4;
+  if (lane < (int)head)
+    dst[lane] = (char)text[lane];
+  const uint32_t r8 = 8u * (head & 3u);
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(text) + (head >> 2);
+  uint4* dv = reinterpret_cast<uint4*>(dst + head);
+  for (uint32_t i = lane; i < body; i += 32) {
+    const uint32_t* w = sw + 4 * i;
+    const uint32_t a0 = w[0], a1 = w[1], a2 = w[2], a3 = w[3], a4 = w[4];
+    dv[i] = make_uint4(__funnelshift_r(a0, a1, r8), __funnelshift_r(a1, a2, r8), __funnelshift_r(a2, a3, r8),
+                       __funnelshift_r(a3, a4, r8));
+  }
+  const uint32_t tail = head + 16u * body + lane;
+  if (tail < len)
+    dst[tail] = (char)text[tail];
+}
+
+__global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedSink out)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  unsigned char* sbuf = smem;                                         // staged text
-  uint8_t* len = smem + kFusedText;                                   // entry lengths, run by run
-  uint16_t* queue = reinterpret_cast<uint16_t*>(len + kFusedTile);    // nonzero entries
-  uint32_t* toff = reinterpret_cast<uint32_t*>(queue + kFusedTile);  // staged offset of each run
-  __shared__ uint32_t qn;
   __shared__ long long s_tile;
   __shared__ unsigned long long s_prefix;
-  __shared__ uint32_t warp_sum[kFusedThreads / 32];
+  __shared__ uint32_t s_len[kFusedWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    qn = 0;
+  WarpText& W = reinterpret_cast<WarpText*>(smem)[warp];
+  if (threadIdx.x == 0)
     s_tile = (long long)atomicAdd(out.ticket, 1u);
-  }
   __syncthreads();
   const long long tile = s_tile;
-  // 1. the run's entries, their +0 / row-end flags and the +0 lengths
-  const int o0 = kRun * (int)threadIdx.x;
-  const long long e0 = tile * kFusedTile + o0;
-  const uint32_t* words = s.ff ? reinterpret_cast<const uint32_t*>(s.ff) : s.counts;
-  uint32_t raw[kRun];
-  if (e0 + kRun <= s.n_entries && ((uintptr_t)(words + e0) & 15u) == 0) {
-    const uint4* p = reinterpret_cast<const uint4*>(words + e0);
+  // 1. the warp's entries, the nonzero ones queued.  n <= 65535: an entry
+  // index fits 32 bits.
+  WarpRows at;
+  const long long first_entry = tile * kFusedTile + (long long)warp * kWarpEntries;
+  at.valid = (int)max(0ll, min((long long)kWarpEntries, s.n_entries - first_entry));
+  at.e0 = at.valid ? (uint32_t)first_entry : 0u;
+  at.n = (uint32_t)s.n;
+  at.row = at.e0 / at.n;
+  at.col = at.e0 - at.row * at.n;
+  const uint32_t* words = (s.ff ? reinterpret_cast<const uint32_t*>(s.ff) : s.counts) + at.e0;
+  uint32_t raw[kChunks];
+  if (at.valid == kWarpEntries) {
 #pragma unroll
-    for (int j = 0; j < kRun / 4; ++j) {
-      const uint4 w = __ldg(p + j);
-      raw[4 * j] = w.x;
-      raw[4 * j + 1] = w.y;
-      raw[4 * j + 2] = w.z;
-      raw[4 * j + 3] = w.w;
-    }
+    for (int k = 0; k < kChunks; ++k)
+      raw[k] = __ldg(words + 32 * k + lane);
   } else {
 #pragma unroll
-    for (int k = 0; k < kRun; ++k)
-      raw[k] = e0 + k < s.n_entries ? __ldg(words + e0 + k) : 0u;
+    for (int k = 0; k < kChunks; ++k)
+      raw[k] = 32 * k + lane < at.valid ? __ldg(words + 32 * k + lane) : 0u;
   }
-  int row = (int)(e0 / s.n), col = (int)(e0 - (long long)row * s.n);
-  float ratio = (!s.ff && row < s.n) ? row_ratio(s, row) : 1.f;
-  uint32_t zero_mask = 0, end_mask = 0, lens[kRun / 4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-  for (int k = 0; k < kRun; ++k) {
-    const bool valid = e0 + k < s.n_entries;
-    const float v = s.ff ? __uint_as_float(raw[k]) : (float)raw[k] * ratio;
-    const bool zero = valid && __float_as_uint(v) == 0u;
-    zero_mask |= zero ? 1u << k : 0u;
-    end_mask |= col == s.n - 1 ? 1u << k : 0u;
-    lens[k >> 2] |= zero ? 2u << (8 * (k & 3)) : 0u;
-    enqueue(queue, &qn, valid && !zero, o0 + k);
-    if (++col == s.n) {
-      col = 0;
-      ++row;
-      if (!s.ff && row < s.n)
-        ratio = row_ratio(s, row);
+  // a count of zero is a +0 entry unless its row's ratio is negative,
+  // infinite or not a number (no rays, or fewer than none)
+  bool plain = true;
+  at.ratio0 = at.ratio1 = 1.f;
+  if (!s.ff && at.valid) {
+    uint32_t r, c;
+    at.locate(at.valid - 1, &r, &c);
+    int rays = 1;
+    for (uint32_t i = at.row + lane; i <= r; i += 32) {
+      rays = __ldg(s.outgoing + i);
+      plain &= rays > 0;
     }
+    plain = __all_sync(0xFFFFFFFFu, plain);
+    const float ratio = 1.f / (float)rays;
+    at.ratio0 = __shfl_sync(0xFFFFFFFFu, ratio, 0);
+    at.ratio1 = __shfl_sync(0xFFFFFFFFu, ratio, 1);
   }
-  *reinterpret_cast<uint4*>(len + o0) = make_uint4(lens[0], lens[1], lens[2], lens[3]);
-  __syncthreads();
-  const uint32_t n_q = qn;
-  for (uint32_t q = threadIdx.x; q < n_q; q += kFusedThreads) {
-    const int o = queue[q];
-    int c;
-    len[o] = (uint8_t)(format_g6_len(fused_value(s, tile, o, &c)) + 1);
-  }
-  __syncthreads();
-  // 2. run lengths, the tile's length and each run's offset in the tile
-  const uint4 lw = *reinterpret_cast<const uint4*>(len + o0);
-  const uint32_t run_len[4] = {lw.x, lw.y, lw.z, lw.w};  // four entry lengths per word
-  const uint32_t mine = __dp4a(lw.x, 0x01010101u, __dp4a(lw.y, 0x01010101u, __dp4a(lw.z, 0x01010101u,
-                                                                                  __dp4a(lw.w, 0x01010101u, 0u))));
-  uint32_t incl = mine;
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-    if (lane >= d)
-      incl += y;
-  }
-  if (lane == 31)
-    warp_sum[warp] = incl;
+  at.simple = plain && at.valid == kWarpEntries && at.n >= (uint32_t)kWarpEntries;
+  at.row_end = (int)(at.n - 1 - at.col);
+  // 2. the nonzero ones formatted, lengths scanned
+  Text first{0, 0, 0};
+  int text_len = 0;
+  const int n_q = at.simple ? queue_entries<true>(s, at, words, raw, plain, W, first, &text_len, lane)
+                            : queue_entries<false>(s, at, words, raw, plain, W, first, &text_len, lane);
+  const uint32_t len = (uint32_t)text_len;
+  if (lane == 0)
+    s_len[warp] = len;
   __syncthreads();
   uint32_t before = 0, total = 0;
-  for (int w = 0; w < kFusedThreads / 32; ++w) {
-    const uint32_t u = warp_sum[w];
+#pragma unroll
+  for (int w = 0; w < kFusedWarps; ++w) {
+    const uint32_t u = s_len[w];
     before += w < warp ? u : 0u;
     total += u;
   }
-  // 3. publish the tile's length; its text is staged from offset 0 while
-  // the tiles before it finish
+  // 3. publish the tile's length; the text is staged while the tiles before
+  // it finish
   if (threadIdx.x == 0)
     st_relaxed(out.status + tile, (tile == 0 ? kTilePrefix : kTileAgg) | total);
-  uint32_t pos = before + incl - mine;
-  toff[threadIdx.x] = pos;
-  if (zero_mask == 0xFFFFu && (pos & 1u) == 0u) {
-    // a run of sixteen +0 entries at an even offset (the common case of a
-    // sparse matrix): its 32 bytes "0;0;...0;" as word stores (a halfword at
-    // each end when the run starts two bytes into a word), then the
-    // newlines of any row ends: 9 or 10 shared stores instead of 32 byte
-    // stores at a 32-byte stride, which put eight lanes on one bank
-    constexpr uint32_t kZeroSemi = 0x3B303B30u;  // "0;0;" little-endian
-    uint32_t p = pos;
-    if (p & 2u) {
-      *reinterpret_cast<uint16_t*>(sbuf + p) = (uint16_t)kZeroSemi;
-      p += 2;
-    }
-    const uint32_t words = (pos + 32u - p) >> 2;
-#pragma unroll 8
-    for (uint32_t w = 0; w < words; ++w)
-      reinterpret_cast<uint32_t*>(sbuf + p)[w] = kZeroSemi;
-    p += 4u * words;
-    if (p < pos + 32u)
-      *reinterpret_cast<uint16_t*>(sbuf + p) = (uint16_t)kZeroSemi;
-    for (uint32_t m = end_mask; m; m &= m - 1u)
-      sbuf[pos + 2u * (uint32_t)(__ffs(m) - 1) + 1u] = '\n';
-  } else {
-#pragma unroll
-    for (int k = 0; k < kRun; ++k) {
-      if ((zero_mask >> k) & 1u) {
-        sbuf[pos] = '0';
-        sbuf[pos + 1] = ((end_mask >> k) & 1u) ? '\n' : ';';
-      }
-      pos += (run_len[k >> 2] >> (8 * (k & 3))) & 0xFFu;
-    }
-  }
-  __syncthreads();
-  for (uint32_t q = threadIdx.x; q < n_q; q += kFusedThreads) {
-    const int o = queue[q];
-    const int t = o / kRun;
-    uint32_t at = toff[t];
-    for (int j = t * kRun; j < o; ++j)
-      at += len[j];
-    int c;
-    const float v = fused_value(s, tile, o, &c);
-    PtrOut w{reinterpret_cast<char*>(sbuf + at), 0};
-    format_g6_to(v, w);
-    w.put(c == s.n - 1 ? '\n' : ';');
-  }
+  const bool fits = len <= (uint32_t)kWindow;
+  if (fits && at.simple)
+    stage_text<true, true>(s, at, words, W, n_q, first, 0, lane);
+  else if (fits)
+    stage_text<true, false>(s, at, words, W, n_q, first, 0, lane);
   // 4. the tile's place in the text
   if (warp == 0) {
     unsigned long long excl = 0;
@@ -871,25 +1094,17 @@ __global__ void __launch_bounds__(kFusedThreads, FFB_CSV_BLOCKS) k_csv_fused(Sou
       atomicOr(out.err, kFusedOverflow);
     return;
   }
-  // 5. copy the staged text to text + P: bytes up to the first 16-byte
-  // boundary, then 16-byte stores assembled from 32-bit shared words
-  // (funnel shifts by the staged offset's misalignment), then the tail
-  char* dst = out.text + P;
-  const uint32_t head = min(total, (uint32_t)((16u - ((uintptr_t)dst & 15u)) & 15u));
-  const uint32_t body = (total - head) >> 4;
-  for (uint32_t i = threadIdx.x; i < head; i += kFusedThreads)
-    dst[i] = (char)sbuf[i];
-  const uint32_t r8 = 8u * (head & 3u);
-  const uint32_t* sw = reinterpret_cast<const uint32_t*>(sbuf) + (head >> 2);
-  uint4* dv = reinterpret_cast<uint4*>(dst + head);
-  for (uint32_t i = threadIdx.x; i < body; i += kFusedThreads) {
-    const uint32_t* w = sw + 4 * i;
-    const uint32_t a0 = w[0], a1 = w[1], a2 = w[2], a3 = w[3], a4 = w[4];
-    dv[i] = make_uint4(__funnelshift_r(a0, a1, r8), __funnelshift_r(a1, a2, r8), __funnelshift_r(a2, a3, r8),
-                       __funnelshift_r(a3, a4, r8));
+  char* dst = out.text + P + before;
+  if (fits) {
+    copy_text(dst, W.text, len, lane);
+    return;
   }
-  for (uint32_t i = head + 16u * body + threadIdx.x; i < total; i += kFusedThreads)
-    dst[i] = (char)sbuf[i];
+  for (uint32_t w0 = 0; w0 < len; w0 += kWindow) {
+    stage_text<false, false>(s, at, words, W, n_q, first, (int)w0, lane);
+    __syncwarp();
+    copy_text(dst + w0, W.text, min(len - w0, (uint32_t)kWindow), lane);
+    __syncwarp();
+  }
 }
 #endif  // __CUDACC__
 
