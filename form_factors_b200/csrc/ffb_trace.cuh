@@ -147,17 +147,18 @@ __device__ __forceinline__ void warp_hash_flush(uint32_t* keys, uint32_t* vals, 
 
 // ---------------------------------------------------------------------------
 // Fused form-factor kernel.  Persistent warps, no block barriers.  Each warp
-// keeps a current chunk (consecutive rays of one face) and hands its rays to
-// lanes as they fall idle (one ballot per refill, one global atomic per
-// chunk), so a warp may hold rays of several faces at once.  Idle lanes are
-// refilled together once at least the shape's `refill` of them wait (or the
-// whole warp is idle): emission and ray setup then run with several lanes at
-// once instead of one lane at a time.  Each iteration a lane whose cell is
-// exhausted moves on (stop, DDA step or empty-space jump; up to the shape's
-// `adv` moves while it lands in empty cells) and then tests up to its `test`
-// references of its cell.  Doing both kinds of work in one
-// iteration keeps lanes of a warp in the same code more of the time than
-// one kind per iteration does.  A finished hit adds one to the
+// keeps a current chunk (consecutive rays of one face; one global atomic per
+// chunk) and emits its next 32 rays, one per lane, into a queue in shared
+// memory whenever the queue is empty.  Idle lanes are refilled from the queue
+// together once at least the shape's `refill` of them wait (or the whole warp
+// is idle), so a warp may hold rays of several faces at once.  Emission by
+// the idle lanes themselves, 6 to 8 of 32, took 15 of 167 warp instructions
+// per ray.  Each iteration a lane tests up to the shape's `test` references
+// of its cell and, when it has none left, moves on (stop, DDA step or
+// empty-space jump; up to `adv` moves while it lands in empty cells): this
+// order took 5 % less than moving before testing.  Letting a vote of the warp
+// pick one kind of work per iteration filled more lanes and was 6 to 11 %
+// slower: it waits for memory more often.  A finished hit adds one to the
 // warp's shared-memory hash histogram keyed by the matrix index
 // row(f) * n_cols + row(h); the warp flushes the table to the global uint32
 // matrix with atomic adds when it is half full and at the end.
@@ -166,14 +167,14 @@ __device__ __forceinline__ void warp_hash_flush(uint32_t* keys, uint32_t* vals, 
 // replaces the matrix: a hit adds the per-ray power of the ray's (source
 // face, side) to the absorbed power of the hit face's mesh, in 64-bit fixed
 // point (integer sums: the same result whatever the order of the hits).
-// kStats adds the test / cell / ray / hit counters (four live registers per
-// lane); without it p.stats is ignored.  kHash selects the warp histogram;
+// kStats adds the test / cell / ray / hit counters (Tally); without it
+// p.stats is ignored.  kHash selects the warp histogram;
 // without it each hit is one global reduction (red.global.add) into the
 // matrix, which suits large, sparse matrices (distinct keys per warp, so the
 // histogram merges little) and leaves the shared memory to the L1 cache.
 // ---------------------------------------------------------------------------
 #ifndef FFB_REFILL_MIN
-#define FFB_REFILL_MIN 6
+#define FFB_REFILL_MIN 8
 #endif
 constexpr int kRefillMin = FFB_REFILL_MIN;
 // cell advances and triangle tests a lane may do per iteration
@@ -279,18 +280,106 @@ __device__ __forceinline__ void direction_order(uint32_t face, uint32_t j0, int 
   __syncwarp();
 }
 
+// The lanes' test / cell / ray / hit / jump counters, in shared memory: five
+// more registers a lane spill.  For 22 M rays in a closed room of 22 080
+// faces they cost 0.7 ms of 6.2; these cost 0.4 of 5.2.
+enum { kCountTests, kCountCells, kCountRays, kCountHits, kCountJumps };
+template <bool kOn>
+struct Tally {
+  uint32_t (*n)[kTraceThreads];
+  __device__ __forceinline__ void clear()
+  {
+    if constexpr (kOn) {
+      __shared__ uint32_t s_count[kCountJumps + 1][kTraceThreads];
+      n = s_count;
+#pragma unroll
+      for (int k = 0; k <= kCountJumps; ++k)
+        n[k][threadIdx.x] = 0;
+    }
+  }
+  __device__ __forceinline__ void add(int k, uint32_t x)
+  {
+    if constexpr (kOn)
+      n[k][threadIdx.x] += x;
+  }
+  __device__ __forceinline__ void flush(unsigned long long* stats)
+  {
+    if constexpr (kOn)
+      warp_stats(stats, n[kCountTests][threadIdx.x], n[kCountCells][threadIdx.x], n[kCountRays][threadIdx.x],
+                 n[kCountHits][threadIdx.x], n[kCountJumps][threadIdx.x]);
+  }
+};
+
+// Part of a lane's state (the first kVectors vectors of Tracer), set aside in
+// local memory around a rare stretch of code that needs many registers: the
+// exact test (one ray in twenty) and the emission of 32 rays.  Left to itself
+// the compiler fits the loop into 64 registers by spilling 84 bytes a thread
+// of what every iteration uses; 80 registers spill nothing but leave six
+// blocks per SM.  22 M rays in a closed room, ms: 5.4 spilling, 5.9 with six
+// blocks, 4.8 with this.  How much to set aside is measured for each variant:
+// more than it takes to end the spills only adds stores.
+template <int kVectors>
+struct TracerHold {
+  volatile float v[3 * kVectors + (kVectors == 0)];
+  __device__ __forceinline__ explicit TracerHold(const Tracer& T)
+  {
+    const float3* a[6] = {&T.og, &T.dg, &T.po, &T.pd, &T.iv, &T.io};
+#pragma unroll
+    for (int k = 0; k < kVectors; ++k) {
+      v[3 * k] = a[k]->x;
+      v[3 * k + 1] = a[k]->y;
+      v[3 * k + 2] = a[k]->z;
+    }
+  }
+  __device__ __forceinline__ void release(Tracer& T) const
+  {
+    float3* a[6] = {&T.og, &T.dg, &T.po, &T.pd, &T.iv, &T.io};
+#pragma unroll
+    for (int k = 0; k < kVectors; ++k)
+      *a[k] = f3(v[3 * k], v[3 * k + 1], v[3 * k + 2]);
+  }
+};
+
+// Tests up to kTest pending references of the cell of each active lane; the
+// ray for the exact test comes from shared memory (`ray`).
+template <int kTest, int kHold, bool kFar>
+__device__ __forceinline__ void warp_tests(Tracer& T, const GridView& g, bool active,
+                                           const float4 (&ray)[2][kTraceThreads], uint32_t& n_tests)
+{
+  if (active && T.i < T.en) {
+    int open = -1;
+#pragma unroll
+    for (int k = 0; k < kTest; ++k)
+      if (T.i < T.en && open < 0)
+        open = tracer_test<kFar>(T, g, n_tests);
+    if (open >= 0) {
+      const TracerHold<kHold> hold(T);
+      const float4 q = ray[0][threadIdx.x], r = ray[1][threadIdx.x];
+      tracer_exact(T, g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
+      hold.release(T);
+    }
+  }
+}
+
 template <bool kStats, bool kHash, bool kPower = false, int kShape = 0>
 __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     k_form_factors(const __grid_constant__ TraceParams p)
 {
   constexpr TraceShape kS = trace_shape(kShape);
+  // vectors set aside around the emission and the exact test (TracerHold)
+  constexpr int kHoldFill = kS.coherent ? 4 : kStats ? 1 : 0, kHoldExact = kStats || kHash ? 6 : 3;
   extern __shared__ uint32_t s_hash[];  // kWarpsPerBlock x (keys, values) when kHash
   // coherent hand-out: per warp, direction-bin counters and the chunk's ray order
   __shared__ uint32_t s_bins[kS.coherent ? kWarpsPerBlock * kDirBins : 1];
   __shared__ uint8_t s_perm[kS.coherent ? kWarpsPerBlock * kChunkRaysMax : 1];
   // each lane's ray for the exact test: (origin, direction x), (direction y, z, start distance, row)
   __shared__ float4 s_ray[2][kTraceThreads];
+  // rays of each warp that are emitted but not handed out: (origin, direction x), (direction y, z, -, row)
+  __shared__ float4 s_queue[2][kTraceThreads];
+  __shared__ int4 s_chunk[kWarpsPerBlock];  // (face, j, front, row)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Tally<kStats> count;
+  count.clear();
   if (p.span && threadIdx.x == 0)
     atomicMin(p.span, global_ns());
   uint32_t* keys = s_hash + warp * 2 * kWarpHash;
@@ -306,7 +395,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
   const unsigned lane_below = (1u << lane) - 1u;
   int fill = 0;  // occupied slots (warp-uniform)
   // current chunk (warp-uniform); c_pos: its rays handed out so far
-  int c_face = 0, c_j = 0, c_left = 0, c_front = 0, c_row = 0, c_pos = 0;
+  int c_left = 0;
   const SceneSlot& S = p.scene;
   uint32_t key0 = p.key0, key1 = p.key1;
   if (p.scene_keys) {
@@ -314,83 +403,103 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     key0 = k.x;
     key1 = k.y;
   }
+  int q_pos = 0, q_end = 0;  // queued rays [q_pos, q_end) (warp-uniform)
   bool exhausted = false;
-  uint32_t n_tests = 0, n_cells = 0, n_rays = 0, n_hits = 0, n_jumps = 0;
   // lane state
   Tracer T;
   bool active = false;
   for (;;) {
     unsigned need = __ballot_sync(kFull, !active);
-
-    if (__popc(need) < kS.refill && need != kFull)
+    if ((__popc(need) < kS.refill && need != kFull) || (exhausted && q_pos == q_end))
       need = 0;
-    while (need && !exhausted) {
-      if (c_left == 0) {
-        int k = 0;
-        if (lane == 0)
-          k = (int)atomicAdd(p.chunk_cursor, 1u);
-        k = __shfl_sync(kFull, k, 0);
-        if (k >= p.n_chunks) {
-          exhausted = true;
-          break;
+    while (need) {
+      if (q_pos == q_end) {
+        // the next 32 rays of the warp's chunks, one per lane (after every
+        // lane has read the last ones)
+        __syncwarp();
+        const TracerHold<kHoldFill> hold(T);
+        q_pos = q_end = 0;
+        while (q_end < 32 && !exhausted) {
+          if (c_left == 0) {
+            int k = 0;
+            if (lane == 0)
+              k = (int)atomicAdd(p.chunk_cursor, 1u);
+            k = __shfl_sync(kFull, k, 0);
+            if (k >= p.n_chunks) {
+              exhausted = true;
+              break;
+            }
+            const Chunk ch = p.chunks[k];
+            c_left = ch.count;
+            if (lane == 0)
+              s_chunk[warp] = make_int4(ch.face, kS.coherent ? ch.j0 : ch.j0 + ch.count, ch.front,
+                                        S.face_to_row ? __ldg(S.face_to_row + ch.face) : ch.face);
+            __syncwarp();
+            if (kS.coherent)
+              direction_order((uint32_t)ch.face, (uint32_t)ch.j0, c_left, key0, key1, epoch, s_bins + warp * kDirBins,
+                              s_perm + warp * kChunkRaysMax, lane);
+          }
+          const int take = min(32 - q_end, c_left), rank = lane - q_end;
+          if (rank >= 0 && rank < take) {
+            const int4 ch = s_chunk[warp];
+            const int c_face = ch.x, c_front = ch.z, c_row = ch.w;
+            const int j =
+                ch.y + (kS.coherent ? (int)s_perm[warp * kChunkRaysMax + c_left - 1 - rank] : rank - c_left);
+            float3 o, e;
+            emit_ray(p.frames + 20 * ((size_t)S.face_base + c_face), (uint32_t)c_face, (uint32_t)j, c_front, key0, key1,
+                     epoch, o, e);
+            count.add(kCountRays, 1u);
+            const float3 dir = sub3(e, o);
+            s_queue[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
+            s_queue[1][threadIdx.x] =
+                make_float4(dir.y, dir.z, 0.f, __int_as_float(kPower ? 2 * c_face + (j >= c_front ? 1 : 0) : c_row));
+          }
+          c_left -= take;
+          q_end += take;
         }
-        const Chunk ch = p.chunks[k];
-        c_face = ch.face;
-        c_j = ch.j0;
-        c_left = ch.count;
-        c_front = ch.front;
-        c_row = S.face_to_row ? __ldg(S.face_to_row + ch.face) : ch.face;
-        c_pos = 0;
-        if (kS.coherent)
-          direction_order((uint32_t)c_face, (uint32_t)c_j, c_left, key0, key1, epoch, s_bins + warp * kDirBins,
-                          s_perm + warp * kChunkRaysMax, lane);
+        __syncwarp();
+        hold.release(T);
+        if (q_end == 0)
+          break;
       }
-      const int take = min(__popc(need), c_left);
+      const int take = min(__popc(need), q_end - q_pos);
       const int rank = __popc(need & lane_below);
       const bool mine = ((need >> lane) & 1u) && rank < take;
       if (mine) {
-        const int j = c_j + (kS.coherent ? (int)s_perm[warp * kChunkRaysMax + c_pos + rank] : c_pos + rank);
-        float3 o, e;
-        emit_ray(p.frames + 20 * ((size_t)S.face_base + c_face), (uint32_t)c_face, (uint32_t)j, c_front, key0, key1,
-                 epoch, o, e);
-        ++n_rays;
-        const float3 dir = sub3(e, o);
-        float t0;
-        active = tracer_begin<false>(T, S.g, o, dir, &t0, n_cells);
-        s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
-        s_ray[1][threadIdx.x] =
-            make_float4(dir.y, dir.z, t0, __int_as_float(kPower ? 2 * c_face + (j >= c_front ? 1 : 0) : c_row));
+        const float4 q = s_queue[0][(threadIdx.x & ~31) + q_pos + rank];
+        float4 r = s_queue[1][(threadIdx.x & ~31) + q_pos + rank];
+        uint32_t n_cells = 0;
+        active = tracer_begin<false>(T, S.g, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), &r.z, n_cells);
+        count.add(kCountCells, n_cells);
+        s_ray[0][threadIdx.x] = q;
+        s_ray[1][threadIdx.x] = r;
       }
       need &= ~__ballot_sync(kFull, mine);
-      c_pos += take;
-      c_left -= take;
+      q_pos += take;
     }
-    if (exhausted && !__any_sync(kFull, active))
+    if (exhausted && q_pos == q_end && !__any_sync(kFull, active))
       break;
-    int hit = -1, open = -1;
-    if (active) {
+    uint32_t n_tests = 0;
+    warp_tests<kS.test, kHoldExact, false>(T, S.g, active, s_ray, n_tests);
+    count.add(kCountTests, n_tests);
+    int hit = -1;
+    if (active && T.i >= T.en) {
       bool live = true;
+      uint32_t n_cells = 0, n_jumps = 0;
 #pragma unroll
       for (int k = 0; k < kS.adv; ++k)
         if (live && T.i >= T.en)
           live = tracer_advance(T, S.g, n_cells, n_jumps);
+      count.add(kCountCells, n_cells);
+      count.add(kCountJumps, n_jumps);
       if (!live) {
         active = false;
         hit = T.face;
-      } else {
-#pragma unroll
-        for (int k = 0; k < kS.test; ++k)
-          if (T.i < T.en && open < 0)
-            open = tracer_test<false>(T, S.g, n_tests);
       }
-    }
-    if (open >= 0) {
-      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
-      tracer_exact(T, S.g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
     }
     bool fresh = false;
     if (hit >= 0) {
-      ++n_hits;
+      count.add(kCountHits, 1u);
       const int col = S.face_to_row ? __ldg(S.face_to_row + hit) : hit;
       const int my_row = __float_as_int(s_ray[1][threadIdx.x].w);
       if (kPower) {
@@ -413,8 +522,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
   }
   if (kHash)
     warp_hash_flush(keys, vals, S.counts, lane);
-  if (kStats)
-    warp_stats(p.stats, n_tests, n_cells, n_rays, n_hits, n_jumps);
+  count.flush(p.stats);
   if (p.span && lane == 0)
     atomicMax(p.span + 1, global_ns());
 }
@@ -439,7 +547,8 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
   __shared__ float4 s_ray[2][kTraceThreads];  // as in k_form_factors
   const int lane = threadIdx.x & 31;
   const unsigned lane_below = (1u << lane) - 1u;
-  uint32_t n_tests = 0, n_cells = 0, n_done = 0, n_hits = 0, n_jumps = 0;
+  Tally<kStats> count;
+  count.clear();
   Tracer T;
   bool active = false;
   bool exhausted = false;
@@ -457,10 +566,12 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
         if (j < n_rays) {
           float3 o, e;
           emit_disc_ray(src, j, key0, key1, epoch, o, e);
-          ++n_done;
+          count.add(kCountRays, 1u);
           const float3 dir = sub3(e, o);
           float t0;
+          uint32_t n_cells = 0;
           active = tracer_begin<true>(T, g, o, dir, &t0, n_cells);
+          count.add(kCountCells, n_cells);
           s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
           s_ray[1][threadIdx.x] = make_float4(dir.y, dir.z, t0, 0.f);
         }
@@ -468,18 +579,23 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     }
     if (exhausted && !__any_sync(kFull, active))
       break;
-    int open = -1;
-    if (active) {
+    uint32_t n_tests = 0;
+    warp_tests<FFB_TEST_PER_ITER, 6, true>(T, g, active, s_ray, n_tests);
+    count.add(kCountTests, n_tests);
+    if (active && T.i >= T.en) {
       bool live = true;
+      uint32_t n_cells = 0, n_jumps = 0;
 #pragma unroll
       for (int k = 0; k < FFB_ADV_PER_ITER; ++k)
         if (live && T.i >= T.en)
           live = tracer_advance(T, g, n_cells, n_jumps);
+      count.add(kCountCells, n_cells);
+      count.add(kCountJumps, n_jumps);
       if (!live) {
         active = false;
         const int h = T.face;
         if (h >= 0) {
-          ++n_hits;
+          count.add(kCountHits, 1u);
           // triangle_normal (math/triangle.cpp:114-119), dot with the direction
           const float* q = faces9 + 9 * (size_t)h;
           const float3 p0 = f3(__ldg(q + 0), __ldg(q + 1), __ldg(q + 2));
@@ -488,20 +604,11 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           const float side = dot3(nrm, src.direction);
           atomicAdd(side_counts + 2 * (size_t)h + (side < 0.f ? 0 : 1), 1u);
         }
-      } else {
-#pragma unroll
-        for (int k = 0; k < FFB_TEST_PER_ITER; ++k)
-          if (T.i < T.en && open < 0)
-            open = tracer_test<true>(T, g, n_tests);
       }
-    }
-    if (open >= 0) {
-      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
-      tracer_exact(T, g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
     }
   }
   if (kStats)
-    warp_stats(stats, n_tests, n_cells, n_done, n_hits, n_jumps);
+    count.flush(stats);
 }
 
 // Materialises rays [0, n_rays) of a disc source (parallel_rays_cpu.cpp:88-106).
@@ -540,7 +647,8 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
   __shared__ float4 s_ray[2][kTraceThreads];  // as in k_form_factors
   const int lane = threadIdx.x & 31;
   const unsigned lane_below = (1u << lane) - 1u;
-  uint32_t n_tests = 0, n_cells = 0, n_done = 0, n_hits = 0, n_jumps = 0;
+  Tally<true> count;
+  count.clear();
   Tracer T;
   bool active = false;
   long id = -1;
@@ -554,8 +662,8 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
       hit_point[3 * i + 1] = pt.y;
       hit_point[3 * i + 2] = pt.z;
     }
-    ++n_done;
-    n_hits += h >= 0;
+    count.add(kCountRays, 1u);
+    count.add(kCountHits, h >= 0);
   };
   for (;;) {
     const unsigned need = __ballot_sync(kFull, !active);
@@ -575,7 +683,9 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           const float3 e = f3(__ldg(q + 3), __ldg(q + 4), __ldg(q + 5));
           const float3 dir = sub3(e, o);
           float t0;
+          uint32_t n_cells = 0;
           active = tracer_begin<true>(T, g, o, dir, &t0, n_cells);
+          count.add(kCountCells, n_cells);
           s_ray[0][threadIdx.x] = make_float4(o.x, o.y, o.z, dir.x);
           s_ray[1][threadIdx.x] = make_float4(dir.y, dir.z, t0, 0.f);
           if (!active)
@@ -585,13 +695,18 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     }
     if (exhausted && !__any_sync(kFull, active))
       break;
-    int open = -1;
-    if (active) {
+    uint32_t n_tests = 0;
+    warp_tests<FFB_TEST_PER_ITER, 6, true>(T, g, active, s_ray, n_tests);
+    count.add(kCountTests, n_tests);
+    if (active && T.i >= T.en) {
       bool live = true;
+      uint32_t n_cells = 0, n_jumps = 0;
 #pragma unroll
       for (int k = 0; k < FFB_ADV_PER_ITER; ++k)
         if (live && T.i >= T.en)
           live = tracer_advance(T, g, n_cells, n_jumps);
+      count.add(kCountCells, n_cells);
+      count.add(kCountJumps, n_jumps);
       if (!live) {
         active = false;
         float3 pt = f3(0.f, 0.f, 0.f);
@@ -600,19 +715,10 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           tri_hit(reinterpret_cast<const float4*>(g.tri + T.face), f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), pt);
         }
         finish(id, T.face, pt);
-      } else {
-#pragma unroll
-        for (int k = 0; k < FFB_TEST_PER_ITER; ++k)
-          if (T.i < T.en && open < 0)
-            open = tracer_test<true>(T, g, n_tests);
       }
     }
-    if (open >= 0) {
-      const float4 q = s_ray[0][threadIdx.x], r = s_ray[1][threadIdx.x];
-      tracer_exact(T, g, open, f3(q.x, q.y, q.z), f3(q.w, r.x, r.y), r.z);
-    }
   }
-  warp_stats(stats, n_tests, n_cells, n_done, n_hits, n_jumps);
+  count.flush(stats);
 }
 
 // Brute force: every ray against every face (the naive_cpu definition),
