@@ -2173,7 +2173,13 @@ int csv_run(ffb_ctx* c, csv::Source src, char* text, unsigned long long cap, FIL
                                 (int)csv::write_smem(csv::kTileBytes)));
   src.n_entries = (long long)src.n * src.n;
   const long long n_tiles = (src.n_entries + csv::kTile - 1) / csv::kTile;
-  const long long n_fused = (src.n_entries + csv::kFusedTile - 1) / csv::kFusedTile;
+  // Entries per warp of the one-pass kernel: 512, or 128 while blocks of 512
+  // would not fill one wave (five per SM).  The text of 637^2 full floats then
+  // takes 39 us instead of 64, of 1500^2 at one nonzero in five 63 for 62, but
+  // of 3000^2 at one in thirty 108 for 67.
+  const bool small = src.n_entries < 5ll * c->n_sm * csv::FusedShape<512>::kTile;
+  const int fused_tile = small ? csv::FusedShape<128>::kTile : csv::FusedShape<512>::kTile;
+  const long long n_fused = (src.n_entries + fused_tile - 1) / fused_tile;
   FFB_TRY(ensure(c, c->csv_tile_len, sizeof(unsigned long long) * (size_t)std::max(n_tiles, n_fused)));
   FFB_TRY(ensure(c, c->csv_tile_off, sizeof(unsigned long long) * (size_t)(n_tiles + 2)));
   auto* tile_len = dptr<unsigned long long>(c->csv_tile_len);
@@ -2184,8 +2190,9 @@ int csv_run(ffb_ctx* c, csv::Source src, char* text, unsigned long long cap, FIL
     // one pass: the tile-length buffer holds the look-back status words; the
     // first two words of the offset buffer the ticket and error bits, then
     // the total
-    FFB_CUDA(cudaFuncSetAttribute(csv::k_csv_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)csv::kFusedSmem));
+    void (*const fused)(csv::Source, csv::FusedSink) = small ? csv::k_csv_fused<128> : csv::k_csv_fused<512>;
+    const size_t fused_smem = small ? csv::FusedShape<128>::kSmem : csv::FusedShape<512>::kSmem;
+    FFB_CUDA(cudaFuncSetAttribute(fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem));
     FFB_CUDA(cudaMemsetAsync(tile_len, 0, sizeof(unsigned long long) * (size_t)n_fused, c->stream));
     FFB_CUDA(cudaMemsetAsync(tile_off, 0, 2 * sizeof(unsigned long long), c->stream));
     csv::FusedSink sink;
@@ -2196,7 +2203,7 @@ int csv_run(ffb_ctx* c, csv::Source src, char* text, unsigned long long cap, FIL
     sink.err = reinterpret_cast<unsigned int*>(tile_off) + 1;
     sink.total = tile_off + 1;
     sink.n_tiles = n_fused;
-    csv::k_csv_fused<<<(unsigned)n_fused, csv::kFusedThreads, csv::kFusedSmem, c->stream>>>(src, sink);
+    fused<<<(unsigned)n_fused, csv::kFusedThreads, fused_smem, c->stream>>>(src, sink);
     FFB_CUDA(cudaGetLastError());
     unsigned long long aux[2] = {0, 0};  // {ticket | err << 32, total}
     FFB_CUDA(cudaMemcpyAsync(aux, tile_off, sizeof aux, cudaMemcpyDeviceToHost, c->stream));

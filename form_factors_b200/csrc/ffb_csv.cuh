@@ -727,7 +727,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_csv_write(Source s, const unsig
 // ---------------------------------------------------------------------------
 // Single pass into a device buffer (decoupled look-back).  Each block takes
 // the next tile by ticket, so every tile it waits for already runs and waits
-// only for earlier tiles.  A warp works through its 512 consecutive entries
+// only for earlier tiles.  A warp works through its 512 (or 128) consecutive entries
 // without block barriers: lane l holds entries 32k + l, ballots give the
 // nonzero ones, which go to the warp's queue in entry order and are formatted
 // by all lanes together; a scan of their lengths gives, for an entry with q
@@ -739,13 +739,15 @@ __global__ void __launch_bounds__(kThreads, 4) k_csv_write(Source s, const unsig
 // buffer writes nothing and sets kFusedOverflow; the last tile writes the text
 // length.
 //
-// What bounds it: instruction issue (about 50 warp instructions per 32
+// What bounds it: instruction issue (about 80 warp instructions per 32
 // entries); 487 M entries of which 4.5 % are nonzero, 1.06 GB of text: 3.34 ms
 // with a whole tile per barrier phase, each nonzero formatted twice by digit
 // loops and zeros staged by byte stores at a 32-byte stride (eight lanes on a
 // bank); 1.73 ms as it is now.  A warp stages 2 KB of text at a time, which
 // holds its 512 entries unless over a fifth of them are nonzero: shared memory
-// for the longest possible text would leave three blocks per SM.
+// for the longest possible text would leave three blocks per SM.  A matrix
+// that would not fill one wave of blocks so takes 128 entries per warp
+// (csv_run).
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kTileAgg = 1ull << 62;     // status: the tile's own length
 constexpr unsigned long long kTilePrefix = 2ull << 62;  // status: the inclusive prefix
@@ -754,19 +756,22 @@ constexpr unsigned kLookbackPolls = 1u << 22;           // polls of one status w
 enum : unsigned { kFusedTimeout = 1u, kFusedOverflow = 2u };
 constexpr int kFusedThreads = 256;
 constexpr int kFusedWarps = kFusedThreads / 32;
-constexpr int kWarpEntries = 512;
-constexpr int kChunks = kWarpEntries / 32;
-constexpr int kFusedTile = kWarpEntries * kFusedWarps;  // entries per tile
-constexpr int kWindow = 2048;                           // staged text per warp, a multiple of 16
 
-// A warp's shared memory.
-struct WarpText {
-  __align__(16) unsigned char text[kWindow + 16];  // one word is read past the window
-  uint16_t entry[kWarpEntries];                    // nonzero entries, in order
-  uint16_t extra[kWarpEntries + 1];                // sum of (length - 2) of those before
-  uint32_t nonzero[kChunks];                       // their lanes in each chunk of 32
+// kEntries: entries per warp, 512 or 128 (csv_run).
+template <int kEntries>
+struct FusedShape {
+  static constexpr int kTile = kEntries * kFusedWarps;  // entries per block
+  // staged text per warp, a multiple of 16
+  static constexpr int kWindow = kEntries * (kMaxEntry - 3) < 2048 ? kEntries * (kMaxEntry - 3) : 2048;
+  // A warp's shared memory.
+  struct WarpText {
+    __align__(16) unsigned char text[kWindow + 16];  // one word is read past the window
+    uint16_t entry[kEntries];                        // nonzero entries, in order
+    uint16_t extra[kEntries + 1];                    // sum of (length - 2) of those before
+    uint32_t nonzero[kEntries / 32];                 // their lanes in each chunk of 32
+  };
+  static constexpr size_t kSmem = sizeof(WarpText) * kFusedWarps;
 };
-constexpr size_t kFusedSmem = sizeof(WarpText) * kFusedWarps;
 
 struct FusedSink {
   char* text;
@@ -822,16 +827,17 @@ __device__ __forceinline__ unsigned long long look_back(const FusedSink& out, lo
   }
 }
 
-// Entries [e0, e0 + 512) of one warp: where they lie in the matrix.
+// Entries [e0, e0 + kEntries) of one warp: where they lie in the matrix.
+template <int kEntries>
 struct WarpRows {
   uint32_t e0;
   uint32_t row, col;  // of entry e0
   uint32_t n;
-  int valid;          // entries before the matrix end, at most 512
+  int valid;          // entries before the matrix end, at most kEntries
 
-  // 512 entries of one or two rows, every count of zero a +0 entry
+  // kEntries entries of one or two rows, every count of zero a +0 entry
   bool simple;
-  int row_end;        // simple: the last entry of the first row (past 511 if it goes on)
+  int row_end;        // simple: the last entry of the first row (past the last if it goes on)
   float ratio0, ratio1;  // simple: of the two rows (counts)
 
   // Separator after entry o, and entry o as text.
@@ -870,7 +876,7 @@ struct WarpRows {
     uint32_t k = col + (uint32_t)o;
     *r = row;
     if (k >= n) {
-      const uint32_t q = n > (uint32_t)kWarpEntries ? 1u : k / n;
+      const uint32_t q = n > (uint32_t)kEntries ? 1u : k / n;
       *r += q;
       k -= q * n;
     }
@@ -881,10 +887,12 @@ struct WarpRows {
 // Stages the warp's text bytes [w0, w0 + kWindow) at W.text; `first` is the
 // text of the lane's first queue entry.  With kAll the whole text fits the
 // window.
-template <bool kAll, bool kSimple>
-__device__ __forceinline__ void stage_text(const Source& s, const WarpRows& at, const uint32_t* words, WarpText& W, int n_q,
-                                           const Text& first, int w0, int lane)
+template <int kEntries, bool kAll, bool kSimple>
+__device__ __forceinline__ void stage_text(const Source& s, const WarpRows<kEntries>& at, const uint32_t* words,
+                                           typename FusedShape<kEntries>::WarpText& W, int n_q, const Text& first,
+                                           int w0, int lane)
 {
+  constexpr int kChunks = kEntries / 32, kWindow = FusedShape<kEntries>::kWindow;
   const uint32_t below = (1u << lane) - 1u;
   const uint16_t* extra = W.extra;  // of the nonzeros in the chunks before
 #pragma unroll 8
@@ -893,7 +901,7 @@ __device__ __forceinline__ void stage_text(const Source& s, const WarpRows& at, 
     const int o = 32 * k + lane;
     if (!((m >> lane) & 1u) && (kSimple || o < at.valid)) {
       const int p = 2 * o + extra[__popc(m & below)] - w0;
-      const unsigned char sep = (unsigned char)at.separator<kSimple>(o);
+      const unsigned char sep = (unsigned char)at.template separator<kSimple>(o);
       if (kAll || (unsigned)p < (unsigned)kWindow)
         W.text[p] = '0';
       if (kAll || (unsigned)(p + 1) < (unsigned)kWindow)
@@ -908,7 +916,7 @@ __device__ __forceinline__ void stage_text(const Source& s, const WarpRows& at, 
       continue;
     Text t = first;
     if (q >= 32)
-      t = at.text<kSimple>(s, words, o);
+      t = at.template text<kSimple>(s, words, o);
     if (kAll) {
       put_bytes(W.text + p, t);
     } else {
@@ -923,11 +931,13 @@ __device__ __forceinline__ void stage_text(const Source& s, const WarpRows& at, 
 // The warp's entries: the nonzero ones queued and formatted (`first` is the
 // text of the lane's first), their lengths scanned.  Returns their number;
 // *len gets the length of the warp's text.
-template <bool kSimple>
-__device__ __forceinline__ int queue_entries(const Source& s, const WarpRows& at, const uint32_t* words,
-                                             const uint32_t (&raw)[kChunks], bool plain, WarpText& W, Text& first,
-                                             int* len, int lane)
+template <int kEntries, bool kSimple>
+__device__ __forceinline__ int queue_entries(const Source& s, const WarpRows<kEntries>& at, const uint32_t* words,
+                                             const uint32_t (&raw)[kEntries / 32], bool plain,
+                                             typename FusedShape<kEntries>::WarpText& W, Text& first, int* len,
+                                             int lane)
 {
+  constexpr int kChunks = kEntries / 32;
   const uint32_t below = (1u << lane) - 1u;
   int n_q = 0;
 #pragma unroll
@@ -952,7 +962,7 @@ __device__ __forceinline__ int queue_entries(const Source& s, const WarpRows& at
     const int q = q0 + lane;
     int mine = 0;
     if (q < n_q) {
-      const Text t = at.text<kSimple>(s, words, W.entry[q]);
+      const Text t = at.template text<kSimple>(s, words, W.entry[q]);
       mine = t.len - 2;
       if (q0 == 0)
         first = t;
@@ -997,8 +1007,11 @@ __device__ __forceinline__ void copy_text(char* dst, const unsigned char* text, 
     dst[tail] = (char)text[tail];
 }
 
+template <int kEntries>
 __global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedSink out)
 {
+  constexpr int kChunks = kEntries / 32, kWindow = FusedShape<kEntries>::kWindow;
+  using WarpText = typename FusedShape<kEntries>::WarpText;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long s_tile;
   __shared__ unsigned long long s_prefix;
@@ -1011,16 +1024,16 @@ __global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedS
   const long long tile = s_tile;
   // 1. the warp's entries, the nonzero ones queued.  n <= 65535: an entry
   // index fits 32 bits.
-  WarpRows at;
-  const long long first_entry = tile * kFusedTile + (long long)warp * kWarpEntries;
-  at.valid = (int)max(0ll, min((long long)kWarpEntries, s.n_entries - first_entry));
+  WarpRows<kEntries> at;
+  const long long first_entry = tile * FusedShape<kEntries>::kTile + (long long)warp * kEntries;
+  at.valid = (int)max(0ll, min((long long)kEntries, s.n_entries - first_entry));
   at.e0 = at.valid ? (uint32_t)first_entry : 0u;
   at.n = (uint32_t)s.n;
   at.row = at.e0 / at.n;
   at.col = at.e0 - at.row * at.n;
   const uint32_t* words = (s.ff ? reinterpret_cast<const uint32_t*>(s.ff) : s.counts) + at.e0;
   uint32_t raw[kChunks];
-  if (at.valid == kWarpEntries) {
+  if (at.valid == kEntries) {
 #pragma unroll
     for (int k = 0; k < kChunks; ++k)
       raw[k] = __ldg(words + 32 * k + lane);
@@ -1046,13 +1059,13 @@ __global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedS
     at.ratio0 = __shfl_sync(0xFFFFFFFFu, ratio, 0);
     at.ratio1 = __shfl_sync(0xFFFFFFFFu, ratio, 1);
   }
-  at.simple = plain && at.valid == kWarpEntries && at.n >= (uint32_t)kWarpEntries;
+  at.simple = plain && at.valid == kEntries && at.n >= (uint32_t)kEntries;
   at.row_end = (int)(at.n - 1 - at.col);
   // 2. the nonzero ones formatted, lengths scanned
   Text first{0, 0, 0};
   int text_len = 0;
-  const int n_q = at.simple ? queue_entries<true>(s, at, words, raw, plain, W, first, &text_len, lane)
-                            : queue_entries<false>(s, at, words, raw, plain, W, first, &text_len, lane);
+  const int n_q = at.simple ? queue_entries<kEntries, true>(s, at, words, raw, plain, W, first, &text_len, lane)
+                            : queue_entries<kEntries, false>(s, at, words, raw, plain, W, first, &text_len, lane);
   const uint32_t len = (uint32_t)text_len;
   if (lane == 0)
     s_len[warp] = len;
@@ -1070,9 +1083,9 @@ __global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedS
     st_relaxed(out.status + tile, (tile == 0 ? kTilePrefix : kTileAgg) | total);
   const bool fits = len <= (uint32_t)kWindow;
   if (fits && at.simple)
-    stage_text<true, true>(s, at, words, W, n_q, first, 0, lane);
+    stage_text<kEntries, true, true>(s, at, words, W, n_q, first, 0, lane);
   else if (fits)
-    stage_text<true, false>(s, at, words, W, n_q, first, 0, lane);
+    stage_text<kEntries, true, false>(s, at, words, W, n_q, first, 0, lane);
   // 4. the tile's place in the text
   if (warp == 0) {
     unsigned long long excl = 0;
@@ -1100,7 +1113,7 @@ __global__ void __launch_bounds__(kFusedThreads, 5) k_csv_fused(Source s, FusedS
     return;
   }
   for (uint32_t w0 = 0; w0 < len; w0 += kWindow) {
-    stage_text<false, false>(s, at, words, W, n_q, first, (int)w0, lane);
+    stage_text<kEntries, false, false>(s, at, words, W, n_q, first, (int)w0, lane);
     __syncwarp();
     copy_text(dst + w0, W.text, min(len - w0, (uint32_t)kWindow), lane);
     __syncwarp();

@@ -66,3 +66,15 @@ def test_counts(ctx, n, rays):
     ff = np.where(np.isnan(ff), np.float32(np.nan), ff).astype(np.float32)  # 0 * inf on the GPU is a positive NaN
     _check(ctx, _text(ff), (3 * n) % 16, counts=torch.from_numpy(counts.view(np.int32)).cuda(),
            outgoing=torch.from_numpy(outgoing).cuda())
+
+
+@pytest.mark.parametrize("n", [1739, 1742, 1793])  # 5 x 148 blocks of 4096 entries: 1741 rows and a part
+def test_sizes_around_one_wave(ctx, n):
+    """The switch from 128 to 512 entries per warp, sparse rows and full ones."""
+    import torch
+    rng = np.random.default_rng(n)
+    ff = np.zeros((n, n), np.float32)
+    m = rng.random((n, n)) < 0.03
+    m[5:40] = True
+    ff[m] = rng.integers(1, 40, int(m.sum())).astype(np.float32) * np.float32(1 / 997)
+    _check(ctx, _text(ff), n % 16, ff=torch.from_numpy(ff).cuda())
