@@ -59,9 +59,11 @@ struct TraceParams {
   unsigned long long* __restrict__ stats;     // kStatSlots, or null
   // radiance sink (kPower): per-ray power of each (face, side) as 64-bit
   // fixed point, and the per-mesh absorbed power it adds to (mesh = the
-  // scene's face_to_row of the hit face)
+  // scene's face_to_row of the hit face), in absorb_mask + 1 copies
+  // absorb_stride apart (k_tally_sum)
   const unsigned long long* __restrict__ power;
   unsigned long long* __restrict__ absorb;
+  uint32_t absorb_mask = 0, absorb_stride = 0;
   // when set: [0] gets the earliest block start and [1] the latest warp end
   // of the launch, in %globaltimer nanoseconds (atomicMin / atomicMax, so
   // several launches may share one pair)
@@ -503,7 +505,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
       const int col = S.face_to_row ? __ldg(S.face_to_row + hit) : hit;
       const int my_row = __float_as_int(s_ray[1][threadIdx.x].w);
       if (kPower) {
-        atomicAdd(p.absorb + col, __ldg(p.power + my_row));
+        atomicAdd(p.absorb + (size_t)(blockIdx.x & p.absorb_mask) * p.absorb_stride + col, __ldg(p.power + my_row));
       } else {
         const uint32_t key = (uint32_t)my_row * (uint32_t)S.n_cols + (uint32_t)col;
         if (kHash)
@@ -542,8 +544,8 @@ template <bool kStats>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_parallel_rays(GridView g, const __grid_constant__ DiscSource src, const float* __restrict__ faces9,
                     unsigned long long n_rays, uint32_t key0, uint32_t key1, uint32_t epoch,
-                    uint32_t* __restrict__ side_counts, unsigned long long* __restrict__ cursor,
-                    unsigned long long* __restrict__ stats)
+                    uint32_t* __restrict__ side_counts, uint32_t copy_mask, uint32_t copy_stride,
+                    unsigned long long* __restrict__ cursor, unsigned long long* __restrict__ stats)
 {
   __shared__ float4 s_ray[2][kTraceThreads], s_queue[2][kTraceThreads];  // as in k_form_factors
   const int lane = threadIdx.x & 31;
@@ -621,13 +623,46 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
           const float3 nrm = cross3(sub3(f3(__ldg(q + 3), __ldg(q + 4), __ldg(q + 5)), p0),
                                     sub3(f3(__ldg(q + 6), __ldg(q + 7), __ldg(q + 8)), p0));
           const float side = dot3(nrm, src.direction);
-          atomicAdd(side_counts + 2 * (size_t)h + (side < 0.f ? 0 : 1), 1u);
+          atomicAdd(side_counts + (size_t)(blockIdx.x & copy_mask) * copy_stride + 2 * (size_t)h + (side < 0.f ? 0 : 1),
+                    1u);
         }
       }
     }
   }
   if (kStats)
     count.flush(stats);
+}
+
+// out[i] = the sum of in[k * stride + i] over `copies` copies, i below n.
+//
+// The sinks with few counters (a distant source's tallies, the radiance
+// equation's meshes) are bound by atomics that meet in the same cache lines:
+// 2.2 M hits on a clutter of 1959 faces took 0.30 to 0.46 ms of which 0.16 to
+// 0.32 went with the atomics taken out.  Blocks so add into several copies of
+// the counters (tally_copies), and this kernel sums them.  Integer sums: the
+// same result in any order.
+constexpr int kSumCounters = 32, kSumLanes = 8;
+template <class T>
+__global__ void __launch_bounds__(kSumCounters* kSumLanes)
+    k_tally_sum(const T* __restrict__ in, int copies, int stride, int n, T* __restrict__ out)
+{
+  __shared__ T part[kSumLanes][kSumCounters];
+  const int x = threadIdx.x % kSumCounters, y = threadIdx.x / kSumCounters;
+  const int i = blockIdx.x * kSumCounters + x;
+  T sum = 0;
+  if (i < n) {
+#pragma unroll 8
+    for (int k = y; k < copies; k += kSumLanes)
+      sum += in[(size_t)k * stride + i];
+  }
+  part[y][x] = sum;
+  __syncthreads();
+  if (y == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < kSumLanes; ++k)
+      sum += part[k][x];
+    out[i] = sum;
+  }
 }
 
 // Materialises rays [0, n_rays) of a disc source (parallel_rays_cpu.cpp:88-106).
