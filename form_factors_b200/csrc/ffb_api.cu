@@ -76,9 +76,16 @@ constexpr int kMaxPipeBlocks = 16;  // row blocks of a pipelined host output
 
 // Host outputs of the count matrix of at least FFB_PIPELINE_MIN_BYTES are
 // traced in row blocks of about FFB_PIPELINE_BLOCK_BYTES (2 to
-// kMaxPipeBlocks) whose copies overlap the next block's trace.
+// kMaxPipeBlocks) whose copies overlap the next block's trace.  Form factors
+// to pageable memory, one launch and a dense copy against row blocks and
+// pairs, for one nonzero in 50 and one in four: 62 MB 3.9 -> 0.7 and 4.5 ->
+// 1.6 ms, 18 MB 1.26 -> 0.36 and 1.50 -> 0.60; to pinned memory 18 MB 0.55 ->
+// 0.37 and 0.76 -> 0.61.  11 MB still gain (0.83 -> 0.30 ms, 0.39 -> 0.30
+// pinned), but a context's first call pays 2 to 5 ms for streams, host threads
+// and pinned memory, which 16 MB make up for in about five calls; from 3 MB
+// down pinned outputs lose.
 #ifndef FFB_PIPELINE_MIN_BYTES
-#define FFB_PIPELINE_MIN_BYTES (64ull << 20)
+#define FFB_PIPELINE_MIN_BYTES (16ull << 20)
 #endif
 #ifndef FFB_PIPELINE_BLOCK_BYTES
 #define FFB_PIPELINE_BLOCK_BYTES (160ull << 20)
@@ -161,10 +168,10 @@ struct ffb_ctx {
   // blocks and their headers, pinned copies of them, and the host threads
   // that expand them into the caller's rows
   DevBuf pack_hdr, pack_pairs;
+  uint32_t* pack_host = nullptr;  // one pinned block: the headers, then two stages
+  size_t pack_host_cap = 0;
   uint32_t* pack_hdr_host = nullptr;
-  size_t pack_hdr_host_cap = 0;
   uint32_t* pack_stage[2] = {nullptr, nullptr};
-  size_t pack_stage_cap = 0;
   int host_threads = -1;  // -1: the default, min(12, hardware threads)
   ffb_host_pool* host_pool = nullptr;
   unsigned long long last_d2h = 0;  // device->host bytes of the last counts call
@@ -857,9 +864,7 @@ extern "C" void ffb_ctx_destroy(ffb_ctx* c)
   for (cudaEvent_t e : c->block_copied)
     if (e) cudaEventDestroy(e);
   ffb_host_pool_destroy(c->host_pool);
-  if (c->pack_hdr_host) cudaFreeHost(c->pack_hdr_host);
-  for (uint32_t* p : c->pack_stage)
-    if (p) cudaFreeHost(p);
+  if (c->pack_host) cudaFreeHost(c->pack_host);
   if (c->pinned_free) cudaEventDestroy(c->pinned_free);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -1155,7 +1160,7 @@ int ensure_pinned(uint32_t** p, size_t* cap, size_t bytes)
 {
   if (bytes <= *cap)
     return FFB_OK;
-  const size_t want = std::max(std::max(bytes, 2 * *cap), (size_t)8 << 20);
+  const size_t want = std::max(std::max(bytes, 2 * *cap), (size_t)1 << 20);
   if (*p)
     cudaFreeHost(*p);
   *p = nullptr;
@@ -1374,28 +1379,35 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   if (packed) {
     size_t& hw = hdr_words;
     size_t pw = 0, max_cap = 0;
+    // an entry that is not zero takes a ray
+    std::vector<size_t> most(n_blocks, 0);
+    for (int b = 0; b < n_blocks; ++b)
+      for (const int32_t f : by_block[b])
+        most[b] += (size_t)std::min<long long>(front[f] + (long long)rear[f], n_rows);
     for (int b = 0; b < n_blocks; ++b) {
       const int rows = bounds[b + 1] - bounds[b];
       hdr_off.push_back(hw);
       pair_off.push_back(pw);
-      cap.push_back((uint32_t)std::min<size_t>((size_t)rows * n_rows / 4, UINT32_MAX));
+      cap.push_back((uint32_t)std::min<size_t>({(size_t)rows * n_rows / 4, most[b], UINT32_MAX}));
       hw += pack_header_words(rows);
       pw += cap.back();
       max_cap = std::max<size_t>(max_cap, cap.back());
     }
     FFB_TRY(ensure(c, c->pack_hdr, sizeof(uint32_t) * hw));
     FFB_TRY(ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1)));
-    FFB_TRY(ensure_pinned(&c->pack_hdr_host, &c->pack_hdr_host_cap, sizeof(uint32_t) * hw));
-    // both stages hold a block's pairs; sized at once for blocks of up to
-    // FFB_PIPELINE_BLOCK_BYTES (the blocks of every matrix below 16 of them)
-    const size_t stage_bytes = std::max(pair_bytes * std::max<size_t>(max_cap, 1),
-                                        (size_t)FFB_PIPELINE_BLOCK_BYTES / 2);
-    size_t stage_cap = c->pack_stage_cap;
-    for (uint32_t*& st : c->pack_stage) {
-      stage_cap = c->pack_stage_cap;  // both stages have the same capacity
-      FFB_TRY(ensure_pinned(&st, &stage_cap, stage_bytes));
-    }
-    c->pack_stage_cap = stage_cap;
+    // Pinned: the headers and two stages, which hold a block's pairs each.  From
+    // 64 MB on sized at once for blocks of up to FFB_PIPELINE_BLOCK_BYTES (the
+    // blocks of every matrix below 16 of them) and any number of rows.  Locking
+    // memory takes 1.2 ms and 0.2 to 0.3 ms per MB: one block, and a smaller
+    // matrix locks what it needs.
+    const bool large = sizeof(uint32_t) * words >= (64u << 20);
+    const size_t hdr_bytes = (std::max(sizeof(uint32_t) * hw, large ? (size_t)1 << 20 : 0) + 255) / 256 * 256;
+    const size_t stage_bytes =
+        (std::max(pair_bytes * max_cap, large ? (size_t)FFB_PIPELINE_BLOCK_BYTES / 2 : 0) + 255) / 256 * 256;
+    FFB_TRY(ensure_pinned(&c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes));
+    c->pack_hdr_host = c->pack_host;
+    for (int k = 0; k < 2; ++k)
+      c->pack_stage[k] = c->pack_host + (hdr_bytes + k * stage_bytes) / sizeof(uint32_t);
   }
   TraceParams p;
   p.frames = dptr<float>(c->frames);
