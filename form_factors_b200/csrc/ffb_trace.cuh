@@ -68,6 +68,7 @@ struct TraceParams {
   // of the launch, in %globaltimer nanoseconds (atomicMin / atomicMax, so
   // several launches may share one pair)
   unsigned long long* __restrict__ span;
+  int default_shape = 0;  // what launch shape 0 stands for (host only)
   SceneSlot scene;
 };
 
@@ -191,7 +192,8 @@ constexpr int kRefillMin = FFB_REFILL_MIN;
 // (ffb_autotune): cell advances and triangle tests a lane may do per
 // iteration, the idle lanes a warp waits for before it refills them, and the
 // resident blocks of 128 threads per SM the kernel is compiled for (which
-// caps its registers at 65536 / (128 * blocks)).  Shape 0 is the default.
+// caps its registers at 65536 / (128 * blocks)).  Shape 0 is the default; where
+// a scene's grid lists few references per face it stands for shape 12.
 // The shape changes only the order in which lanes do their work, never a
 // ray's result or the counts.
 // With `coherent` set, a warp hands out the rays of each chunk it takes in
