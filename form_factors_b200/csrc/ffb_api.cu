@@ -644,7 +644,8 @@ int chunk_rays(const ffb_ctx* c, long long total)
 // Copies of a sink of n counters of `elem` bytes that `adds` atomic adds go
 // to (k_tally_sum), a power of two.  Each copy starts on a cache line.  More
 // copies while every counter still gets 16 adds on average in each of them
-// (the sum reads them all), up to 2 MB in all and one per four blocks.  6 M
+// (the sum reads them all), up to 2 MB in all and one per four blocks.  Where
+// the context's budget has no room for them, one copy does.  6 M
 // rays absorbed by 10 meshes: 2.06 ms with one copy, 0.84 with 256; 4 M source
 // rays at 300 faces 0.50 and 0.13; 10 M at 20 000 faces the same either way.
 struct TallyCopies {
@@ -1384,7 +1385,8 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   const size_t pair_bytes = narrow ? sizeof(uint32_t) : sizeof(uint2);
   std::vector<size_t> hdr_off, pair_off;
   std::vector<uint32_t> cap;
-  size_t hdr_words = 0;
+  size_t hdr_words = 0, hdr_bytes = 0, stage_bytes = 0;
+  const bool large = sizeof(uint32_t) * words >= (64u << 20);
   c->last_d2h = 0;
   if (packed) {
     size_t& hw = hdr_words;
@@ -1403,18 +1405,24 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
       pw += cap.back();
       max_cap = std::max<size_t>(max_cap, cap.back());
     }
-    FFB_TRY(ensure(c, c->pack_hdr, sizeof(uint32_t) * hw));
-    FFB_TRY(ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1)));
     // Pinned: the headers and two stages, which hold a block's pairs each.  From
     // 64 MB on sized at once for blocks of up to FFB_PIPELINE_BLOCK_BYTES (the
     // blocks of every matrix below 16 of them) and any number of rows.  Locking
     // memory takes 1.2 ms and 0.2 to 0.3 ms per MB: one block, and a smaller
     // matrix locks what it needs.
-    const bool large = sizeof(uint32_t) * words >= (64u << 20);
-    const size_t hdr_bytes = (std::max(sizeof(uint32_t) * hw, large ? (size_t)1 << 20 : 0) + 255) / 256 * 256;
-    const size_t stage_bytes =
+    hdr_bytes = (std::max(sizeof(uint32_t) * hw, large ? (size_t)1 << 20 : 0) + 255) / 256 * 256;
+    stage_bytes =
         (std::max(pair_bytes * max_cap, large ? (size_t)FFB_PIPELINE_BLOCK_BYTES / 2 : 0) + 255) / 256 * 256;
-    FFB_TRY(ensure_pinned(&c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes));
+    int rc = ensure(c, c->pack_hdr, sizeof(uint32_t) * hw);
+    if (rc == FFB_OK)
+      rc = ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1));
+    if (rc == FFB_OK)
+      rc = ensure_pinned(&c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
+    if (rc != FFB_OK && (large || fs))
+      return rc;
+    packed = rc == FFB_OK;  // no room for the pairs: dense blocks
+  }
+  if (packed) {
     c->pack_hdr_host = c->pack_host;
     for (int k = 0; k < 2; ++k)
       c->pack_stage[k] = c->pack_host + (hdr_bytes + k * stage_bytes) / sizeof(uint32_t);
@@ -1677,7 +1685,13 @@ extern "C" int ffb_form_factors(ffb_ctx* c, const int32_t* front, const int32_t*
       inv[(size_t)m] = 1.f / (float)outgoing[m];
     FFB_TRY(upload(c, c->front_dev, outgoing, sizeof(int32_t) * (size_t)n_rows));
     FloatSink fs{ff, inv.data(), dptr<int32_t>(c->front_dev), nullptr};
-    return counts_rows_impl(c, front, rear, seed, epoch, flags, face_to_row, n_rows, 0, n_rows, nullptr, &fs);
+    const int rc =
+        counts_rows_impl(c, front, rear, seed, epoch, flags, face_to_row, n_rows, 0, n_rows, nullptr, &fs);
+    if ((rc != FFB_ERR_NO_MEMORY && rc != FFB_ERR_CUDA) || sizeof(float) * mat >= (64u << 20))
+      return rc;
+    // no room for the pairs or their pinned stages: dense, in the same memory
+    release(c, c->tmp_out);
+    release(c, c->pack_pairs);
   }
   FFB_TRY(ensure(c, c->ff_counts, sizeof(uint32_t) * mat));
   FFB_TRY(ffb_form_factor_counts(c, front, rear, seed, epoch, flags, face_to_row, n_rows,
@@ -1731,9 +1745,13 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
   long long n_chunks = 0;
   FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, total), face_first, &n_chunks, true));
   // the copies, then their sums
-  const TallyCopies tally = tally_copies(total, n_meshes, sizeof(unsigned long long));
-  const size_t n_tally = tally.copies > 1 ? (size_t)tally.copies * tally.stride : (size_t)n_meshes;
-  FFB_TRY(ensure(c, c->absorb, sizeof(unsigned long long) * (n_tally + n_meshes)));
+  TallyCopies tally = tally_copies(total, n_meshes, sizeof(unsigned long long));
+  size_t n_tally = (size_t)tally.copies * tally.stride;
+  if (tally.copies == 1 || ensure(c, c->absorb, sizeof(unsigned long long) * (n_tally + n_meshes)) != FFB_OK) {
+    tally = {1, 0};
+    n_tally = (size_t)n_meshes;
+    FFB_TRY(ensure(c, c->absorb, sizeof(unsigned long long) * n_tally));
+  }
   auto* absorb = dptr<unsigned long long>(c->absorb);
   FFB_CUDA(cudaMemsetAsync(absorb, 0, sizeof(unsigned long long) * n_tally, c->stream));
   FFB_TRY(ensure(c, c->stats, sizeof(unsigned long long) * kStatSlots));
@@ -1838,13 +1856,14 @@ extern "C" int ffb_parallel_rays(ffb_ctx* c, const ffb_disc_source* src, long lo
   void* d_counts;
   bool host_out;
   FFB_TRY(output_ptr(c, side_counts, bytes, c->tmp_out, &d_counts, &host_out));
-  const TallyCopies tally = tally_copies(n_rays, 2ll * s.n_faces, sizeof(uint32_t));
+  TallyCopies tally = tally_copies(n_rays, 2ll * s.n_faces, sizeof(uint32_t));
   uint32_t* d_tally = (uint32_t*)d_counts;
-  size_t tally_bytes = bytes;
-  if (tally.copies > 1) {
-    tally_bytes = sizeof(uint32_t) * (size_t)tally.copies * tally.stride;
-    FFB_TRY(ensure(c, c->absorb, tally_bytes));
+  size_t tally_bytes = sizeof(uint32_t) * (size_t)tally.copies * tally.stride;
+  if (tally.copies > 1 && ensure(c, c->absorb, tally_bytes) == FFB_OK) {
     d_tally = dptr<uint32_t>(c->absorb);
+  } else {
+    tally = {1, 0};
+    tally_bytes = bytes;
   }
   FFB_CUDA(cudaMemsetAsync(d_tally, 0, tally_bytes, c->stream));
   FFB_TRY(ensure(c, c->stats, sizeof(unsigned long long) * kStatSlots));

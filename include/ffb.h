@@ -98,7 +98,7 @@ unsigned long long ffb_ctx_bytes(ffb_ctx* ctx);
  * such counters. */
 int ffb_ctx_set_stats(ffb_ctx* ctx, int on);
 /* Host threads of the context (-1: the default, min(12, hardware threads);
- * 0 to 256).  A count matrix written to a host buffer in row blocks (64 MB
+ * 0 to 256).  A count matrix written to a host buffer in row blocks (16 MB
  * or more, ffb_form_factor_counts(_rows)) crosses PCIe as the (column, count)
  * pairs of each block's nonzero entries, packed on the device, and these
  * threads expand them into the caller's rows with streaming stores while the
@@ -436,13 +436,14 @@ typedef struct {
   int refill_min;     /* idle lanes a warp waits for before it refills them */
   int blocks_per_sm;  /* resident 128-thread blocks per SM the kernel is built for */
   int coherent;       /* 1: a chunk's rays are handed out in direction order */
-  int lanes;          /* 0: one ray per lane in registers; K: K rays per lane in shared memory, one
-                         body (advances or tests) per iteration chosen by a vote of the lanes */
+  int lanes;          /* rays a lane keeps in shared memory: 0 in every shape (one ray, in registers) */
 } ffb_trace_shape;
 
 int ffb_trace_shape_count(void);
 int ffb_trace_shape_get(int shape, ffb_trace_shape* out);
-/* Launch shape of the context's form-factor traces (default 0). */
+/* Launch shape of the context's form-factor traces (default 0, which stands
+ * for shape 12 in scenes whose grid lists fewer than twelve references per
+ * face: three tests per iteration instead of two). */
 int ffb_ctx_set_trace_shape(ffb_ctx* ctx, int shape);
 int ffb_ctx_trace_shape(ffb_ctx* ctx);
 
