@@ -349,6 +349,10 @@ GridView make_view(SceneData& s)
 // (parallel plates 5 to 9), up to 6 % slower in those above (clutter).
 int default_shape(const SceneData& s) { return s.info.n_refs < 12ll * s.info.n_live_faces ? 12 : 0; }
 
+// Whether a scene's test records are read past the L1 cache (ldg8): when they
+// are larger than it.
+bool stream_records(const SceneData& s) { return s.info.n_refs * (long long)sizeof(TestRec) >= 256 << 10; }
+
 int check_ctx(ffb_ctx* c)
 {
   if (!c)
@@ -740,11 +744,23 @@ int check_counts(int n_faces, const int32_t* front, const int32_t* rear, long lo
 #endif
 
 // The timed kernel variant (no counters, matrix sink) for each launch shape.
-template <bool kHash, int... S>
+template <bool kHash, bool kStream, int... S>
 void (*shaped_kernel(int shape, std::integer_sequence<int, S...>))(TraceParams)
 {
-  static void (*const table[])(TraceParams) = {k_form_factors<false, kHash, false, S>...};
+  static void (*const table[])(TraceParams) = {k_form_factors<false, kHash, false, S, kStream>...};
   return table[shape];
+}
+
+// The variant for a launch.
+template <bool kStream>
+void (*fused_kernel(const TraceParams& p, bool hash, int shape))(TraceParams)
+{
+  if (p.power)  // radiance sink: no matrix, no histogram
+    return p.stats ? k_form_factors<true, false, true, 0, kStream> : k_form_factors<false, false, true, 0, kStream>;
+  if (p.stats)
+    return hash ? k_form_factors<true, true, false, 0, kStream> : k_form_factors<true, false, false, 0, kStream>;
+  constexpr std::make_integer_sequence<int, kNumShapes> shapes{};
+  return hash ? shaped_kernel<true, kStream>(shape, shapes) : shaped_kernel<false, kStream>(shape, shapes);
 }
 
 // Occupancy-sized persistent launch of the fused kernel for p.n_chunks
@@ -758,18 +774,10 @@ int launch_fused(ffb_ctx* c, const TraceParams& p, bool timed, cudaStream_t stre
     shape = c->trace_shape;
   if (shape == 0)
     shape = p.default_shape;
-  bool hash = (unsigned long long)p.scene.n_cols * (unsigned long long)p.scene.n_cols < FFB_DIRECT_MIN_WORDS;
-  void (*kern)(TraceParams);
-  if (p.stats)
-    kern = hash ? k_form_factors<true, true> : k_form_factors<true, false>;
-  else if (hash)
-    kern = shaped_kernel<true>(shape, std::make_integer_sequence<int, kNumShapes>{});
-  else
-    kern = shaped_kernel<false>(shape, std::make_integer_sequence<int, kNumShapes>{});
-  if (p.power) {  // radiance sink: no matrix, no histogram
-    kern = p.stats ? k_form_factors<true, false, true> : k_form_factors<false, false, true>;
-    hash = false;
-  }
+  const bool hash =
+      !p.power && (unsigned long long)p.scene.n_cols * (unsigned long long)p.scene.n_cols < FFB_DIRECT_MIN_WORDS;
+  void (*kern)(TraceParams) =
+      p.stream_records ? fused_kernel<true>(p, hash, shape) : fused_kernel<false>(p, hash, shape);
   const size_t smem = hash ? kHashSmem : 0;
   int per_sm = 0;
   FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, smem));
@@ -1058,7 +1066,7 @@ int cast_impl(ffb_ctx* c, const float* rays6, long long n_rays, int32_t* hit_fac
     GridView g = make_view(s);
     FFB_TRY(ensure(c, c->ray_cursor, sizeof(unsigned long long)));
     FFB_CUDA(cudaMemsetAsync(c->ray_cursor.ptr, 0, sizeof(unsigned long long), c->stream));
-    auto kern = k_cast;
+    auto kern = stream_records(s) ? k_cast<true> : k_cast<false>;
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const int blocks = grid_blocks(n_rays, kTraceThreads, std::max(1, per_sm) * c->n_sm);
@@ -1440,6 +1448,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   p.span = nullptr;
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
+  p.stream_records = stream_records(s);
   // the kernel adds at row * n_rows + col; the output holds rows from
   // row_begin, so its base is moved back by row_begin rows (only rows of the
   // range are ever written)
@@ -1594,6 +1603,7 @@ int ffb_trace_prepare(ffb_ctx* c, const int32_t* front, const int32_t* rear, uin
   p.span = dptr<unsigned long long>(c->span);
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
+  p.stream_records = stream_records(s);
   p.scene.counts = counts;
   p.scene.face_to_row = nullptr;
   p.scene.face_base = 0;
@@ -1778,6 +1788,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
     p.absorb_stride = tally.stride;
     p.span = nullptr;
     p.scene.g = make_view(s);
+    p.stream_records = stream_records(s);
     p.scene.counts = nullptr;
     p.scene.face_to_row = dptr<int32_t>(c->rows);
     p.scene.face_base = 0;
@@ -1873,7 +1884,8 @@ extern "C" int ffb_parallel_rays(ffb_ctx* c, const ffb_disc_source* src, long lo
   if (n_rays) {
     const GridView g = make_view(s);
     const bool stats = c->stats_on;
-    auto kern = stats ? k_parallel_rays<true> : k_parallel_rays<false>;
+    auto kern = stream_records(s) ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<false, true>)
+                                  : (stats ? k_parallel_rays<true, false> : k_parallel_rays<false, false>);
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const long long wave = (long long)std::max(per_sm, 1) * c->n_sm;
@@ -2636,6 +2648,7 @@ extern "C" int ffb_batch_launch(ffb_ctx* c, uint32_t* counts, const unsigned lon
     SceneSlot& slot = p.scene;
     slot.g = make_view(c->batch[s]);
     p.default_shape = default_shape(c->batch[s]);
+    p.stream_records = stream_records(c->batch[s]);
     slot.counts = counts + counts_offsets[s];
     slot.face_to_row = nullptr;
     slot.face_base = (int)c->batch_offsets[s];

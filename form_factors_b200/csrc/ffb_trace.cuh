@@ -68,7 +68,8 @@ struct TraceParams {
   // of the launch, in %globaltimer nanoseconds (atomicMin / atomicMax, so
   // several launches may share one pair)
   unsigned long long* __restrict__ span;
-  int default_shape = 0;  // what launch shape 0 stands for (host only)
+  int default_shape = 0;        // what launch shape 0 stands for (host only)
+  bool stream_records = false;  // test records bypass the L1 cache, see ldg8 (host only)
   SceneSlot scene;
 };
 
@@ -171,7 +172,7 @@ __device__ __forceinline__ void warp_hash_flush(uint32_t* keys, uint32_t* vals, 
 // face, side) to the absorbed power of the hit face's mesh, in 64-bit fixed
 // point (integer sums: the same result whatever the order of the hits).
 // kStats adds the test / cell / ray / hit counters (Tally); without it
-// p.stats is ignored.  kHash selects the warp histogram;
+// p.stats is ignored.  kStream: see ldg8.  kHash selects the warp histogram;
 // without it each hit is one global reduction (red.global.add) into the
 // matrix, which suits large, sparse matrices (distinct keys per warp, so the
 // histogram merges little) and leaves the shared memory to the L1 cache.
@@ -353,7 +354,7 @@ struct TracerHold {
 
 // Tests up to kTest pending references of the cell of each active lane; the
 // ray for the exact test comes from shared memory (`ray`).
-template <int kTest, int kHold, bool kFar>
+template <int kTest, int kHold, bool kFar, bool kStream>
 __device__ __forceinline__ void warp_tests(Tracer& T, const GridView& g, bool active,
                                            const float4 (&ray)[2][kTraceThreads], uint32_t& n_tests)
 {
@@ -362,7 +363,7 @@ __device__ __forceinline__ void warp_tests(Tracer& T, const GridView& g, bool ac
 #pragma unroll
     for (int k = 0; k < kTest; ++k)
       if (T.i < T.en && open < 0)
-        open = tracer_test<kFar>(T, g, n_tests);
+        open = tracer_test<kFar, kStream>(T, g, n_tests);
     if (open >= 0) {
       const TracerHold<kHold> hold(T);
       const float4 q = ray[0][threadIdx.x], r = ray[1][threadIdx.x];
@@ -372,7 +373,7 @@ __device__ __forceinline__ void warp_tests(Tracer& T, const GridView& g, bool ac
   }
 }
 
-template <bool kStats, bool kHash, bool kPower = false, int kShape = 0>
+template <bool kStats, bool kHash, bool kPower, int kShape, bool kStream>
 __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     k_form_factors(const __grid_constant__ TraceParams p)
 {
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
     if (exhausted && q_pos == q_end && !__any_sync(kFull, active))
       break;
     uint32_t n_tests = 0;
-    warp_tests<kS.test, kHoldExact, false>(T, S.g, active, s_ray, n_tests);
+    warp_tests<kS.test, kHoldExact, false, kStream>(T, S.g, active, s_ray, n_tests);
     count.add(kCountTests, n_tests);
     int hit = -1;
     if (active && T.i >= T.en) {
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
 // reference chooses the front absorbance) and to side_counts[2h + 1]
 // otherwise.
 // ---------------------------------------------------------------------------
-template <bool kStats>
+template <bool kStats, bool kStream>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_parallel_rays(GridView g, const __grid_constant__ DiscSource src, const float* __restrict__ faces9,
                     unsigned long long n_rays, uint32_t key0, uint32_t key1, uint32_t epoch,
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     if (exhausted && q_pos == q_end && !__any_sync(kFull, active))
       break;
     uint32_t n_tests = 0;
-    warp_tests<FFB_TEST_PER_ITER, 4, true>(T, g, active, s_ray, n_tests);
+    warp_tests<FFB_TEST_PER_ITER, 4, true, kStream>(T, g, active, s_ray, n_tests);
     count.add(kCountTests, n_tests);
     if (active && T.i >= T.en) {
       bool live = true;
@@ -702,6 +703,7 @@ __global__ void k_epoch_bump(uint32_t* epoch)
 // hit_point (optional) gets the point, NaN for a miss.  Persistent warps take
 // rays from a global cursor (one atomic per refill) as lanes fall idle.
 // ---------------------------------------------------------------------------
+template <bool kStream>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_cast(GridView g, const float* __restrict__ rays6, long n_rays, int32_t* __restrict__ hit_face,
            float* __restrict__ hit_point, unsigned long long* __restrict__ stats,
@@ -759,7 +761,7 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     if (exhausted && !__any_sync(kFull, active))
       break;
     uint32_t n_tests = 0;
-    warp_tests<FFB_TEST_PER_ITER, 6, true>(T, g, active, s_ray, n_tests);
+    warp_tests<FFB_TEST_PER_ITER, 6, true, kStream>(T, g, active, s_ray, n_tests);
     count.add(kCountTests, n_tests);
     if (active && T.i >= T.en) {
       bool live = true;
