@@ -130,6 +130,7 @@ struct ffb_ctx {
   int batch_frames_mode = -1;
   int batch_n_chunks = 0;
   std::vector<int> batch_chunk_first;  // first chunk of each scene (scene-major), plus the total
+  std::vector<std::pair<long long, long long>> batch_rays;  // rays and emitting faces of each scene
   std::vector<int> batch_shape;        // launch shape of each scene (ffb_batch_autotune), default 0
   // side streams of the batched launch: one launch per scene, spread over
   // them so that a scene's launch tail overlaps the next scenes
@@ -349,9 +350,18 @@ GridView make_view(SceneData& s)
 // (parallel plates 5 to 9), up to 6 % slower in those above (clutter).
 int default_shape(const SceneData& s) { return s.info.n_refs < 12ll * s.info.n_live_faces ? 12 : 0; }
 
-// Whether a scene's test records are read past the L1 cache (ldg8): when they
-// are larger than it.
-bool stream_records(const SceneData& s) { return s.info.n_refs * (long long)sizeof(TestRec) >= 256 << 10; }
+// Whether a launch of `rays` rays from `faces` faces reads a scene's test
+// records past the L1 cache (ldg8): when they are larger than it and no face
+// emits so many rays that the whole GPU traces a few faces at a time, whose
+// records then are found in L1 (and, read past it, meet in the same L2 lines).
+// Seven scenes of 1280 to 22 080 faces at two grids each: 500 to 8000 rays per
+// face 1 to 19 % faster past L1, 30 000 from 4 % faster to 26 % slower, 100 000
+// up to 2.2 times slower.  Rays cast from memory stay cached: their order is
+// not known.
+bool stream_records(const SceneData& s, long long rays, long long faces)
+{
+  return s.info.n_refs * (long long)sizeof(TestRec) >= 256 << 10 && rays <= 10000 * faces;
+}
 
 int check_ctx(ffb_ctx* c)
 {
@@ -1066,7 +1076,7 @@ int cast_impl(ffb_ctx* c, const float* rays6, long long n_rays, int32_t* hit_fac
     GridView g = make_view(s);
     FFB_TRY(ensure(c, c->ray_cursor, sizeof(unsigned long long)));
     FFB_CUDA(cudaMemsetAsync(c->ray_cursor.ptr, 0, sizeof(unsigned long long), c->stream));
-    auto kern = stream_records(s) ? k_cast<true> : k_cast<false>;
+    auto kern = k_cast;
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const int blocks = grid_blocks(n_rays, kTraceThreads, std::max(1, per_sm) * c->n_sm);
@@ -1448,7 +1458,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   p.span = nullptr;
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
-  p.stream_records = stream_records(s);
+  p.stream_records = stream_records(s, emitted, (long long)order.size());
   // the kernel adds at row * n_rows + col; the output holds rows from
   // row_begin, so its base is moved back by row_begin rows (only rows of the
   // range are ever written)
@@ -1603,7 +1613,7 @@ int ffb_trace_prepare(ffb_ctx* c, const int32_t* front, const int32_t* rear, uin
   p.span = dptr<unsigned long long>(c->span);
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
-  p.stream_records = stream_records(s);
+  p.stream_records = stream_records(s, total, (long long)order.size());
   p.scene.counts = counts;
   p.scene.face_to_row = nullptr;
   p.scene.face_base = 0;
@@ -1788,7 +1798,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
     p.absorb_stride = tally.stride;
     p.span = nullptr;
     p.scene.g = make_view(s);
-    p.stream_records = stream_records(s);
+    p.stream_records = stream_records(s, total, (long long)order.size());
     p.scene.counts = nullptr;
     p.scene.face_to_row = dptr<int32_t>(c->rows);
     p.scene.face_base = 0;
@@ -1884,8 +1894,8 @@ extern "C" int ffb_parallel_rays(ffb_ctx* c, const ffb_disc_source* src, long lo
   if (n_rays) {
     const GridView g = make_view(s);
     const bool stats = c->stats_on;
-    auto kern = stream_records(s) ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<false, true>)
-                                  : (stats ? k_parallel_rays<true, false> : k_parallel_rays<false, false>);
+    auto kern = stream_records(s, 0, 0) ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<false, true>)
+                                        : (stats ? k_parallel_rays<true, false> : k_parallel_rays<false, false>);
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
     const long long wave = (long long)std::max(per_sm, 1) * c->n_sm;
@@ -2527,6 +2537,7 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
   std::vector<int4> src, tail;
   src.reserve((size_t)n_all);
   c->batch_chunk_first.assign(n_scenes + 1, 0);
+  c->batch_rays.assign(n_scenes, {0, 0});
   long long next = 0;
   for (int s = 0; s < n_scenes; ++s) {
     const long long f0 = c->batch_offsets[s];
@@ -2547,9 +2558,11 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
       (is_tail ? tail : src).push_back(make_int4(f, front[f0 + f], (int)nf, (int)next));
       next += (nf + per - 1) / per;
       rays += nf;
+      ++c->batch_rays[s].second;
       if (next > INT_MAX)
         return fail(FFB_ERR_TOO_LARGE, "more than %d work chunks", INT_MAX);
     }
+    c->batch_rays[s].first = rays;
   }
   c->batch_chunk_first[n_scenes] = (int)next;
   c->batch_n_chunks = (int)next;
@@ -2648,7 +2661,7 @@ extern "C" int ffb_batch_launch(ffb_ctx* c, uint32_t* counts, const unsigned lon
     SceneSlot& slot = p.scene;
     slot.g = make_view(c->batch[s]);
     p.default_shape = default_shape(c->batch[s]);
-    p.stream_records = stream_records(c->batch[s]);
+    p.stream_records = stream_records(c->batch[s], c->batch_rays[s].first, c->batch_rays[s].second);
     slot.counts = counts + counts_offsets[s];
     slot.face_to_row = nullptr;
     slot.face_base = (int)c->batch_offsets[s];

@@ -756,7 +756,8 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 // than the hits save: with 0.26 to 28 MB of records 60 of 60 grids traced 2 to
 // 22 % faster without (the room at 162^3 cells 4.80 -> 4.63 ms, plates of
 // 10 000 faces 1.32 -> 1.10 ms).  Smaller tables are found in L1, and need it:
-// 0.05 to 0.2 MB of records up to 1.6 times slower without.
+// 0.05 to 0.2 MB of records up to 1.6 times slower without.  So do launches
+// whose rays start at few faces (stream_records).
 template <bool kStream>
 __device__ __forceinline__ void ldg8(const void* p, float* v)
 {

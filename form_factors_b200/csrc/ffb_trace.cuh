@@ -703,7 +703,6 @@ __global__ void k_epoch_bump(uint32_t* epoch)
 // hit_point (optional) gets the point, NaN for a miss.  Persistent warps take
 // rays from a global cursor (one atomic per refill) as lanes fall idle.
 // ---------------------------------------------------------------------------
-template <bool kStream>
 __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     k_cast(GridView g, const float* __restrict__ rays6, long n_rays, int32_t* __restrict__ hit_face,
            float* __restrict__ hit_point, unsigned long long* __restrict__ stats,
@@ -761,7 +760,7 @@ __global__ void __launch_bounds__(kTraceThreads, FFB_MIN_BLOCKS)
     if (exhausted && !__any_sync(kFull, active))
       break;
     uint32_t n_tests = 0;
-    warp_tests<FFB_TEST_PER_ITER, 6, true, kStream>(T, g, active, s_ray, n_tests);
+    warp_tests<FFB_TEST_PER_ITER, 6, true, false>(T, g, active, s_ray, n_tests);
     count.add(kCountTests, n_tests);
     if (active && T.i >= T.en) {
       bool live = true;
