@@ -734,18 +734,28 @@ struct Tracer {
   uint32_t oct;      // octant of the direction
 };
 
+// Built as plain C++ (a check of the walk on the CPU) the three functions with
+// GPU instructions take a few lines of C++ instead.
 __device__ __forceinline__ float rcp_approx(float x)
 {
+#ifdef __CUDA_ARCH__
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+#else
+  return fabsf(x) < 0x1p-126f ? copysignf(INFINITY, x) : 1.f / x;
+#endif
 }
 
 __device__ __forceinline__ float rsqrt_approx(float x)
 {
+#ifdef __CUDA_ARCH__
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+#else
+  return fabsf(x) < 0x1p-126f ? copysignf(INFINITY, x) : 1.f / sqrtf(x);
+#endif
 }
 
 // 256-bit read-only load (32-byte aligned).  With kStream the line does not
@@ -761,6 +771,9 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 template <bool kStream>
 __device__ __forceinline__ void ldg8(const void* p, float* v)
 {
+#ifndef __CUDA_ARCH__
+  memcpy(v, p, 8 * sizeof(float));
+#else
   if constexpr (kStream)
     asm("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
@@ -769,6 +782,7 @@ __device__ __forceinline__ void ldg8(const void* p, float* v)
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
         : "l"(p));
+#endif
 }
 
 // Reads the record of the current cell: its references, or its empty-space
@@ -789,6 +803,18 @@ __device__ __forceinline__ void tracer_enter(Tracer& T, const GridView& g)
 // Cells of padding before and after the cell table: one index step beyond
 // either end of each axis.
 __host__ __device__ inline long long cell_pad(int nx, int ny) { return 1ll + nx + (long long)nx * ny; }
+
+// Speed of the walk along an axis, cells per world unit; one so small that a
+// plane's distance (up to 256 cells and a jump of 127 over the speed) might
+// overflow counts as zero, whose reciprocal is infinite: the axis is then never
+// stepped and drops out of the minima as a NaN.  Over the diagonal of a box of
+// 2^64, past which squared edges overflow in the reference's test, the ray
+// moves 2^-53 cells along it, far below the landing bias.
+__device__ __forceinline__ float walk_speed(float d)
+{
+  const float a = fabsf(d);
+  return a >= 0x1p-117f ? a : 0.f;
+}
 
 // Sets up the ray o + t dir; false when it misses the grid box (no hit
 // possible).  *t0 gets the distance from o to the point the walk starts at (0
@@ -821,7 +847,7 @@ __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float
   float3 om = f3(mx ? g.nf.x - T.og.x : T.og.x, my ? g.nf.y - T.og.y : T.og.y, mz ? g.nf.z - T.og.z : T.og.z);
   if (!(om.x <= g.nf.x && om.y <= g.nf.y && om.z <= g.nf.z))
     return false;  // beyond the far side of an axis (or not a number)
-  T.pd = f3(fabsf(T.dg.x), fabsf(T.dg.y), fabsf(T.dg.z));
+  T.pd = f3(walk_speed(T.dg.x), walk_speed(T.dg.y), walk_speed(T.dg.z));
   T.iv = f3(rcp_approx(T.pd.x), rcp_approx(T.pd.y), rcp_approx(T.pd.z));
   T.io = f3(-om.x * T.iv.x, -om.y * T.iv.y, -om.z * T.iv.z);
   T.far = 1.f;
