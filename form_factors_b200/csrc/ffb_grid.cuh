@@ -730,7 +730,7 @@ struct Tracer {
   uint32_t i, en;    // pending references of the current cell
   int face;          // best hit, -1 if none
   int sx, sy, sz;    // signed cell strides
-  int base;          // cell index offset
+  uint32_t base;     // cell index offset
   uint32_t oct;      // octant of the direction
 };
 
@@ -791,8 +791,10 @@ __device__ __forceinline__ void ldg8(const void* p, float* v)
 // (cell_pad) below and above, and nothing lies within two margins of the box.
 __device__ __forceinline__ void tracer_enter(Tracer& T, const GridView& g)
 {
-  const int cell = T.base + __float_as_int(T.bx) * T.sx + __float_as_int(T.by) * T.sy + __float_as_int(T.bz) * T.sz;
-  const uint2 r = __ldg(g.cell_rec + cell);
+  // modulo 2^32: the products of the bias overflow and cancel against the base
+  const uint32_t cell = T.base + __float_as_uint(T.bx) * (uint32_t)T.sx + __float_as_uint(T.by) * (uint32_t)T.sy +
+                        __float_as_uint(T.bz) * (uint32_t)T.sz;
+  const uint2 r = __ldg(g.cell_rec + (int)cell);
   const bool empty = (int)r.y < 0;
   const uint32_t d = (__byte_perm(r.x, r.y, T.oct) & 0x7Fu) | 0x4B000000u;  // the octant's byte as 2^23 + d
   T.jump = (empty ? __uint_as_float(d) : 8388609.f) - (8388608.f + kBias);
@@ -876,8 +878,8 @@ __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float
   T.sx = mx ? -1 : 1;
   T.sy = my ? -g.nx : g.nx;
   T.sz = mz ? -g.nxy : g.nxy;
-  T.base = (mx ? g.nxm : 0) + (my ? g.nym : 0) + (mz ? g.nzm : 0) -
-           (int)((uint32_t)kBiasBits * (uint32_t)(T.sx + T.sy + T.sz));
+  T.base = (uint32_t)((mx ? g.nxm : 0) + (my ? g.nym : 0) + (mz ? g.nzm : 0)) -
+           kBiasBits * (uint32_t)(T.sx + T.sy + T.sz);
   T.oct = (mx ? 1u : 0u) | (my ? 2u : 0u) | (mz ? 4u : 0u);
   T.bx = __fadd_rd(T.po.x, kBias);
   T.by = __fadd_rd(T.po.y, kBias);
