@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_shape(kShape).blocks)
             }
             const Chunk ch = p.chunks[k];
             c_left = ch.count;
+            __syncwarp();  // every lane has read the chunk before (a shuffle orders no memory)
             if (lane == 0)
               s_chunk[warp] = make_int4(ch.face, kS.coherent ? ch.j0 : ch.j0 + ch.count, ch.front,
                                         S.face_to_row ? __ldg(S.face_to_row + ch.face) : ch.face);
