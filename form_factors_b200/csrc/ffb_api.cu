@@ -47,12 +47,16 @@ int fail(int code, const char* fmt, ...)
   return code;
 }
 
+// Reports a failed CUDA call, and clears the runtime's last error: the check
+// after a later launch would report it again.
 #define FFB_CUDA(call)                                                                                   \
   do {                                                                                                   \
     cudaError_t e_ = (call);                                                                             \
-    if (e_ != cudaSuccess)                                                                               \
+    if (e_ != cudaSuccess) {                                                                             \
+      cudaGetLastError();                                                                                \
       return fail(e_ == cudaErrorMemoryAllocation ? FFB_ERR_NO_MEMORY : FFB_ERR_CUDA, "%s: %s (%s:%d)", \
                   #call, cudaGetErrorString(e_), __FILE__, __LINE__);                                    \
+    }                                                                                                    \
   } while (0)
 
 #define FFB_TRY(expr)   \
@@ -171,6 +175,7 @@ struct ffb_ctx {
   DevBuf pack_hdr, pack_pairs;
   uint32_t* pack_host = nullptr;  // one pinned block: the headers, then two stages
   size_t pack_host_cap = 0;
+  unsigned long long pinned_limit = 0;  // tests: larger pinned allocations fail (0: none does)
   uint32_t* pack_hdr_host = nullptr;
   uint32_t* pack_stage[2] = {nullptr, nullptr};
   int host_threads = -1;  // -1: the default, min(12, hardware threads)
@@ -264,10 +269,12 @@ int stage(ffb_ctx* c, size_t bytes, void** out)
   if (bytes > c->pinned_cap) {
     if (c->pinned)
       cudaFreeHost(c->pinned);
+    const size_t had = c->pinned_cap;
     c->pinned = nullptr;
+    c->pinned_cap = 0;
     // at least 8 MiB, doubling: page-locked allocations synchronise the
     // device, so the staging buffer grows rarely
-    size_t want = std::max(std::max(bytes, c->pinned_cap * 2), (size_t)8 << 20);
+    size_t want = std::max(std::max(bytes, had * 2), (size_t)8 << 20);
     FFB_CUDA(cudaMallocHost(&c->pinned, want));
     c->pinned_cap = want;
   }
@@ -416,8 +423,10 @@ int ensure_pipeline(ffb_ctx* c)
   }
   if (e == cudaSuccess)
     e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return fail(FFB_ERR_CUDA, "copy stream/event creation: %s", cudaGetErrorString(e));
+  }
   return FFB_OK;
 }
 
@@ -443,8 +452,10 @@ int ensure_batch_streams(ffb_ctx* c)
       e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e == cudaSuccess)
     e = cudaEventCreateWithFlags(&c->batch_fork, cudaEventDisableTiming);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return fail(FFB_ERR_CUDA, "batch stream/event creation: %s", cudaGetErrorString(e));
+  }
   return FFB_OK;
 }
 
@@ -835,6 +846,7 @@ extern "C" int ffb_ctx_create(int device, ffb_ctx** out)
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     delete c;
     return fail(FFB_ERR_CUDA, "stream/event creation: %s", cudaGetErrorString(e));
   }
@@ -1185,11 +1197,13 @@ bool sparse_enough(int n_faces, const int32_t* front, const int32_t* rear, const
 // Pinned host memory of at least `bytes` in *p (capacity *cap), kept and
 // grown by doubling (page-locking costs tens of ms per hundred MB, so a
 // run of growing requests must not pay it each time).
-int ensure_pinned(uint32_t** p, size_t* cap, size_t bytes)
+int ensure_pinned(const ffb_ctx* c, uint32_t** p, size_t* cap, size_t bytes)
 {
   if (bytes <= *cap)
     return FFB_OK;
-  const size_t want = std::max(std::max(bytes, 2 * *cap), (size_t)1 << 20);
+  size_t want = std::max(std::max(bytes, 2 * *cap), (size_t)1 << 20);
+  if (c->pinned_limit && want > c->pinned_limit)
+    want = (size_t)1 << 62;  // more than any address space: the allocation fails as one too large for the host does
   if (*p)
     cudaFreeHost(*p);
   *p = nullptr;
@@ -1278,6 +1292,8 @@ int fetch_packed(ffb_ctx* c, const std::vector<int>& bounds, int row_begin, int 
 }
 
 }  // namespace
+
+void ffb_test_pinned_limit(ffb_ctx* c, unsigned long long bytes) { c->pinned_limit = bytes; }
 
 namespace {
 
@@ -1435,7 +1451,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
     if (rc == FFB_OK)
       rc = ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1));
     if (rc == FFB_OK)
-      rc = ensure_pinned(&c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
+      rc = ensure_pinned(c, &c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
     if (rc != FFB_OK && (large || fs))
       return rc;
     packed = rc == FFB_OK;  // no room for the pairs: dense blocks

@@ -9,6 +9,10 @@
 // Records an error for ffb_last_error and returns `code`.
 int ffb_set_error(int code, const char* msg);
 
+// For tests: pinned allocations of a context's packed host outputs above
+// `bytes` fail as they do on a host that cannot lock so much (0: none fails).
+extern "C" void ffb_test_pinned_limit(ffb_ctx* c, unsigned long long bytes);
+
 // Sliced traces, for the serving loop.  ffb_trace_prepare readies one fused
 // form-factor trace of the context's scene (grid built) with per-face
 // (front, rear) ray counts, Philox (seed, epoch) and emission flags: it

@@ -1,0 +1,45 @@
+"""Host outputs on a host that cannot page-lock memory for them: outputs below
+64 MB, which need none, are written all the same; a larger one reports the failed
+allocation, and that error is gone for the calls after it.  Tolerance: none."""
+import numpy as np
+import pytest
+
+from form_factors_b200 import native, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _limit(ctx, n_bytes):
+    import ctypes
+    fn = native.load().ffb_test_pinned_limit
+    fn.argtypes, fn.restype = [ctypes.c_void_p, ctypes.c_ulonglong], None
+    fn(ctx._h, n_bytes)
+
+
+def test_outputs_without_pinned_memory():
+    faces = np.concatenate([scenes.icosphere(4, 1.0, inward=True)] * 2)[:4400]
+    n, small = len(faces), 2300
+    rays = np.full(n, 60, np.int32)
+    zero = np.zeros(n, np.int32)
+
+    def solve(c, n, factors):
+        return (c.form_factors if factors else c.form_factor_counts)(rays[:n], zero[:n], 9)
+
+    free, tight = native.Context(0), native.Context(0)
+    _limit(tight, 1)
+    for c in (free, tight):
+        c.scene_set(faces[:small])
+        c.grid_build(cells_per_face=16)
+    for factors in (False, True):
+        assert np.array_equal(solve(tight, small, factors), solve(free, small, factors))
+    for c in (free, tight):
+        c.scene_set(faces)
+        c.grid_build(cells_per_face=16)
+    assert n * n * 4 >= 64 << 20
+    want = solve(free, n, False)
+    with pytest.raises(native.FFBError, match="memory"):
+        solve(tight, n, False)
+    _limit(tight, 0)
+    assert np.array_equal(solve(tight, n, False), want)
+    _limit(tight, 1 << 30)
+    assert np.array_equal(solve(tight, n, True), solve(free, n, True))
