@@ -1299,10 +1299,11 @@ namespace {
 
 // ffb_form_factor_counts_rows; with fs, the output is fs's host float
 // matrix of normalised form factors instead of `counts` (a packed host
-// output: the caller checks that it is one).
+// output: the caller checks that it is one).  *launched is set before the
+// first launch.
 int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint64_t seed, uint32_t epoch, int flags,
                      const int32_t* face_to_row, int n_rows, int row_begin, int row_end, uint32_t* counts,
-                     const FloatSink* fs)
+                     const FloatSink* fs, bool* launched = nullptr)
 {
   FFB_TRY(check_ctx(c));
   SceneData& s = c->main;
@@ -1452,6 +1453,12 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
       rc = ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1));
     if (rc == FFB_OK)
       rc = ensure_pinned(c, &c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
+    if (rc == FFB_OK && fs) {  // dense blocks are normalised into a device block before their copy
+      size_t max_words = 0;
+      for (int b = 0; b < n_blocks; ++b)
+        max_words = std::max(max_words, (size_t)(bounds[b + 1] - bounds[b]) * n_rows);
+      rc = ensure(c, c->tmp_out2, sizeof(float) * max_words);
+    }
     if (rc != FFB_OK && (large || fs))
       return rc;
     packed = rc == FFB_OK;  // no room for the pairs: dense blocks
@@ -1490,59 +1497,68 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   // launch tail (a block holds a few chunks per warp) overlaps the next
   // block's launch; blocks share nothing they write (rows, cursor, pairs).
   constexpr int kBlockStreams = 2;
-  if (n_blocks > 1) {
+  if (n_blocks > 1)
     FFB_TRY(ensure_batch_streams(c));
-    FFB_CUDA(cudaEventRecord(c->batch_fork, c->stream));
-    for (int k = 0; k < kBlockStreams; ++k)
-      FFB_CUDA(cudaStreamWaitEvent(c->batch_streams[k], c->batch_fork, 0));
-  }
-  for (int b = 0; b < n_blocks; ++b) {
-    cudaStream_t st = n_blocks > 1 ? c->batch_streams[b % kBlockStreams] : c->stream;
-    const size_t off = (size_t)(bounds[b] - row_begin) * n_rows;
-    const size_t n_words = (size_t)(bounds[b + 1] - bounds[b]) * n_rows;
-    FFB_CUDA(cudaMemsetAsync((uint32_t*)d_counts + off, 0, sizeof(uint32_t) * n_words, st));
-    if (first[b + 1] > first[b]) {
-      p.chunks = dptr<Chunk>(c->chunks) + first[b];
-      p.n_chunks = first[b + 1] - first[b];
-      p.chunk_cursor = dptr<uint32_t>(c->cursor) + b;
-      FFB_TRY(launch_fused(c, p, false, st));
+  const auto launch_blocks = [&]() -> int {
+    if (n_blocks > 1) {
+      FFB_CUDA(cudaEventRecord(c->batch_fork, c->stream));
+      for (int k = 0; k < kBlockStreams; ++k)
+        FFB_CUDA(cudaStreamWaitEvent(c->batch_streams[k], c->batch_fork, 0));
     }
-    if (packed && bounds[b + 1] > bounds[b]) {
-      const int rows = bounds[b + 1] - bounds[b];
-      (narrow ? k_rows_pack<true> : k_rows_pack<false>)<<<std::min(rows, c->n_sm * 8), kPackThreads, 0, st>>>(
-          (const uint32_t*)d_counts + off, rows, n_rows, dptr<uint32_t>(c->pack_hdr) + hdr_off[b], cap[b],
-          dptr<unsigned char>(c->pack_pairs) + pair_bytes * pair_off[b]);
-      FFB_CUDA(cudaGetLastError());
+    for (int b = 0; b < n_blocks; ++b) {
+      cudaStream_t st = n_blocks > 1 ? c->batch_streams[b % kBlockStreams] : c->stream;
+      const size_t off = (size_t)(bounds[b] - row_begin) * n_rows;
+      const size_t n_words = (size_t)(bounds[b + 1] - bounds[b]) * n_rows;
+      FFB_CUDA(cudaMemsetAsync((uint32_t*)d_counts + off, 0, sizeof(uint32_t) * n_words, st));
+      if (first[b + 1] > first[b]) {
+        p.chunks = dptr<Chunk>(c->chunks) + first[b];
+        p.n_chunks = first[b + 1] - first[b];
+        p.chunk_cursor = dptr<uint32_t>(c->cursor) + b;
+        FFB_TRY(launch_fused(c, p, false, st));
+      }
+      if (packed && bounds[b + 1] > bounds[b]) {
+        const int rows = bounds[b + 1] - bounds[b];
+        (narrow ? k_rows_pack<true> : k_rows_pack<false>)<<<std::min(rows, c->n_sm * 8), kPackThreads, 0, st>>>(
+            (const uint32_t*)d_counts + off, rows, n_rows, dptr<uint32_t>(c->pack_hdr) + hdr_off[b], cap[b],
+            dptr<unsigned char>(c->pack_pairs) + pair_bytes * pair_off[b]);
+        FFB_CUDA(cudaGetLastError());
+      }
+      if (n_blocks > 1)
+        FFB_CUDA(cudaEventRecord(c->block_done[b], st));
     }
-    if (n_blocks > 1)
-      FFB_CUDA(cudaEventRecord(c->block_done[b], st));
-  }
-  if (n_blocks > 1)  // the context stream continues after every block
-    for (int k = 0; k < kBlockStreams; ++k) {
-      FFB_CUDA(cudaEventRecord(c->batch_join[k], c->batch_streams[k]));
-      FFB_CUDA(cudaStreamWaitEvent(c->stream, c->batch_join[k], 0));
+    if (n_blocks > 1)  // the context stream continues after every block
+      for (int k = 0; k < kBlockStreams; ++k) {
+        FFB_CUDA(cudaEventRecord(c->batch_join[k], c->batch_streams[k]));
+        FFB_CUDA(cudaStreamWaitEvent(c->stream, c->batch_join[k], 0));
+      }
+    return FFB_OK;
+  };
+  // After an error nothing may still run on the other streams, into buffers
+  // that the next call frees or the caller's memory.
+  const auto drained = [&](int rc) -> int {
+    if (rc != FFB_OK && n_blocks > 1) {
+      for (int k = 0; k < kBlockStreams; ++k)
+        cudaStreamSynchronize(c->batch_streams[k]);
+      cudaStreamSynchronize(c->copy_stream);
+      cudaStreamSynchronize(c->stream);
+      cudaGetLastError();
     }
+    return rc;
+  };
+  if (launched)
+    *launched = true;
+  FFB_TRY(drained(launch_blocks()));
   timing_end(c);
   if (!host_out)
     return FFB_OK;
   if (packed) {
     FloatSink sink;
-    if (fs) {  // dense blocks are normalised into a device block before their copy
-      size_t max_words = 0;
-      for (int b = 0; b < n_blocks; ++b)
-        max_words = std::max(max_words, (size_t)(bounds[b + 1] - bounds[b]) * n_rows);
-      FFB_TRY(ensure(c, c->tmp_out2, sizeof(float) * max_words));
+    if (fs) {
       sink = *fs;
       sink.scratch = dptr<float>(c->tmp_out2);
     }
-    const int rc = fetch_packed(c, bounds, row_begin, n_rows, (const uint32_t*)d_counts, counts, hdr_off, pair_off,
-                                cap, narrow, fs ? &sink : nullptr);
-    if (rc != FFB_OK) {  // nothing may still write into the caller's buffer once the call returns
-      cudaStreamSynchronize(c->copy_stream);
-      cudaStreamSynchronize(c->stream);
-      cudaGetLastError();
-      return rc;
-    }
+    FFB_TRY(drained(fetch_packed(c, bounds, row_begin, n_rows, (const uint32_t*)d_counts, counts, hdr_off, pair_off,
+                                 cap, narrow, fs ? &sink : nullptr)));
   } else if (n_blocks == 1) {
     c->last_d2h = sizeof(uint32_t) * words;
     FFB_TRY(finish_output(c, counts, d_counts, sizeof(uint32_t) * words));
@@ -1550,17 +1566,21 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
     c->last_d2h = sizeof(uint32_t) * words;
     // all launches are queued before the first copy: a copy to pageable
     // memory holds the host until it ends
-    for (int b = 0; b < n_blocks; ++b) {
-      const size_t off = (size_t)(bounds[b] - row_begin) * n_rows;
-      const size_t n_words = (size_t)(bounds[b + 1] - bounds[b]) * n_rows;
-      FFB_CUDA(cudaStreamWaitEvent(c->copy_stream, c->block_done[b], 0));
-      FFB_CUDA(cudaMemcpyAsync(counts + off, (const uint32_t*)d_counts + off, sizeof(uint32_t) * n_words,
-                               cudaMemcpyDeviceToHost, c->copy_stream));
-    }
-    // later work on the context stream (a reuse of the device output) waits
-    // for the copies
-    FFB_CUDA(cudaEventRecord(c->copies_done, c->copy_stream));
-    FFB_CUDA(cudaStreamWaitEvent(c->stream, c->copies_done, 0));
+    const auto copy_blocks = [&]() -> int {
+      for (int b = 0; b < n_blocks; ++b) {
+        const size_t off = (size_t)(bounds[b] - row_begin) * n_rows;
+        const size_t n_words = (size_t)(bounds[b + 1] - bounds[b]) * n_rows;
+        FFB_CUDA(cudaStreamWaitEvent(c->copy_stream, c->block_done[b], 0));
+        FFB_CUDA(cudaMemcpyAsync(counts + off, (const uint32_t*)d_counts + off, sizeof(uint32_t) * n_words,
+                                 cudaMemcpyDeviceToHost, c->copy_stream));
+      }
+      // later work on the context stream (a reuse of the device output) waits
+      // for the copies
+      FFB_CUDA(cudaEventRecord(c->copies_done, c->copy_stream));
+      FFB_CUDA(cudaStreamWaitEvent(c->stream, c->copies_done, 0));
+      return FFB_OK;
+    };
+    FFB_TRY(drained(copy_blocks()));
   }
   FFB_CUDA(cudaStreamSynchronize(c->stream));
   return FFB_OK;
@@ -1721,11 +1741,13 @@ extern "C" int ffb_form_factors(ffb_ctx* c, const int32_t* front, const int32_t*
       inv[(size_t)m] = 1.f / (float)outgoing[m];
     FFB_TRY(upload(c, c->front_dev, outgoing, sizeof(int32_t) * (size_t)n_rows));
     FloatSink fs{ff, inv.data(), dptr<int32_t>(c->front_dev), nullptr};
+    bool launched = false;
     const int rc =
-        counts_rows_impl(c, front, rear, seed, epoch, flags, face_to_row, n_rows, 0, n_rows, nullptr, &fs);
-    if ((rc != FFB_ERR_NO_MEMORY && rc != FFB_ERR_CUDA) || sizeof(float) * mat >= (64u << 20))
+        counts_rows_impl(c, front, rear, seed, epoch, flags, face_to_row, n_rows, 0, n_rows, nullptr, &fs, &launched);
+    if (launched || (rc != FFB_ERR_NO_MEMORY && rc != FFB_ERR_CUDA) || sizeof(float) * mat >= (64u << 20))
       return rc;
-    // no room for the pairs or their pinned stages: dense, in the same memory
+    // nothing ran yet, for want of memory (or streams) for the row blocks:
+    // dense, in the same memory
     release(c, c->tmp_out);
     release(c, c->pack_pairs);
   }

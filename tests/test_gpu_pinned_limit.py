@@ -43,3 +43,22 @@ def test_outputs_without_pinned_memory():
     assert np.array_equal(solve(tight, n, False), want)
     _limit(tight, 1 << 30)
     assert np.array_equal(solve(tight, n, True), solve(free, n, True))
+
+
+def test_factors_without_room_for_dense_blocks():
+    """A budget that holds the pairs of the row blocks but not the block that a
+    dense one would be normalised in: nothing is launched before that is known."""
+    n = 2200
+    faces = scenes.icosphere(4, 1.0, inward=True)[:2 * n:2]
+    front, zero = np.full(n, 540, np.int32), np.zeros(n, np.int32)
+    front[0] = 70000  # pairs of two words: half the matrix
+    free, tight = native.Context(0), native.Context(0)
+    for c in (free, tight):
+        c.scene_set(faces)
+        c.grid_build(cells_per_face=16)
+        c.form_factor_counts(front, zero, 1)
+    before, matrix = tight.device_bytes(), 4 * n * n
+    tight.set_budget(before + int(0.58 * matrix))
+    assert np.array_equal(tight.form_factors(front, zero, 9), free.form_factors(front, zero, 9))
+    assert tight.device_bytes() - before > 0.4 * matrix  # two dense matrices for one and the pairs
+    assert np.array_equal(tight.form_factors(front, zero, 10), free.form_factors(front, zero, 10))
