@@ -76,20 +76,27 @@ constexpr int kChunkRays = 256;  // rays per work chunk of the fused kernel at m
 constexpr int kTailRays = 64;    // rays per chunk of a launch's last sixteenth at most
 static_assert(kChunkRays == kChunkRaysMax, "the coherent hand-out orders whole chunks");
 constexpr int kMaxRows = 65535;  // matrix index row * n + col stays below 0xFFFFFFFF
+constexpr size_t kStageMinBytes = 8 << 20;  // pinned staging buffer of a context
 constexpr int kMaxPipeBlocks = 16;  // row blocks of a pipelined host output
 
 // Host outputs of the count matrix of at least FFB_PIPELINE_MIN_BYTES are
 // traced in row blocks of about FFB_PIPELINE_BLOCK_BYTES (2 to
 // kMaxPipeBlocks) whose copies overlap the next block's trace.  Form factors
 // to pageable memory, one launch and a dense copy against row blocks and
-// pairs, for one nonzero in 50 and one in four: 62 MB 3.9 -> 0.7 and 4.5 ->
-// 1.6 ms, 18 MB 1.26 -> 0.36 and 1.50 -> 0.60; to pinned memory 18 MB 0.55 ->
-// 0.37 and 0.76 -> 0.61.  11 MB still gain (0.83 -> 0.30 ms, 0.39 -> 0.30
-// pinned), but a context's first call pays 2 to 5 ms for streams, host threads
-// and pinned memory, which 16 MB make up for in about five calls; from 3 MB
-// down pinned outputs lose.
+// pairs, for one nonzero in a hundred and one in four: 65 MB 3.5 -> 0.7 and 5.3
+// -> 1.4 ms, 17 MB 1.15 -> 0.38 and 1.7 -> 0.6; to pinned memory 65 MB 1.5 ->
+// 0.7 and 3.3 -> 1.4 ms, 17 MB 0.6 -> 0.37 and 1.15 -> 0.6.  A context's first
+// call, which also makes streams and host threads, gains too: 65 MB 4.5 -> 2.0
+// and 6.1 -> 2.8 ms, 17 MB 1.6 -> 1.1 and 2.3 -> 1.6.  11 MB would still gain
+// on repeated calls; from 3 MB down pinned outputs lose.
 #ifndef FFB_PIPELINE_MIN_BYTES
 #define FFB_PIPELINE_MIN_BYTES (16ull << 20)
+#endif
+// From here on a context locks memory for an output's pairs (1.2 ms and 0.2 to
+// 1 ms per MB, for what the rays bound the pairs by: 31 ms in the first call of
+// 1.95 GB at 1000 rays a row, 100 with stages for any block).
+#ifndef FFB_PINNED_MIN_BYTES
+#define FFB_PINNED_MIN_BYTES (64ull << 20)
 #endif
 #ifndef FFB_PIPELINE_BLOCK_BYTES
 #define FFB_PIPELINE_BLOCK_BYTES (160ull << 20)
@@ -173,7 +180,7 @@ struct ffb_ctx {
   // blocks and their headers, pinned copies of them, and the host threads
   // that expand them into the caller's rows
   DevBuf pack_hdr, pack_pairs;
-  uint32_t* pack_host = nullptr;  // one pinned block: the headers, then two stages
+  uint32_t* pack_host = nullptr;  // one pinned block: the headers, then two stages (FFB_PINNED_MIN_BYTES)
   size_t pack_host_cap = 0;
   unsigned long long pinned_limit = 0;  // tests: larger pinned allocations fail (0: none does)
   uint32_t* pack_hdr_host = nullptr;
@@ -272,9 +279,9 @@ int stage(ffb_ctx* c, size_t bytes, void** out)
     const size_t had = c->pinned_cap;
     c->pinned = nullptr;
     c->pinned_cap = 0;
-    // at least 8 MiB, doubling: page-locked allocations synchronise the
-    // device, so the staging buffer grows rarely
-    size_t want = std::max(std::max(bytes, had * 2), (size_t)8 << 20);
+    // at least kStageMinBytes, doubling: page-locked allocations synchronise
+    // the device, so the staging buffer grows rarely
+    size_t want = std::max(std::max(bytes, had * 2), kStageMinBytes);
     FFB_CUDA(cudaMallocHost(&c->pinned, want));
     c->pinned_cap = want;
   }
@@ -1159,10 +1166,6 @@ extern "C" int ffb_emit(ffb_ctx* c, const int32_t* front, const int32_t* rear, u
 
 namespace {
 
-// Whether rows [row_begin, row_end) of the count matrix are sparse enough
-// for the packed transfer: a row holds at most min(its rays, n_rows)
-// nonzero entries, and the bound summed over the rows must fit the pair
-// caps (a quarter of the entries).  Denser matrices go dense as a whole.
 // The context's host threads, started (or restarted with a new count) on
 // first use; false when they cannot be started.
 bool ensure_host_pool(ffb_ctx* c)
@@ -1182,16 +1185,28 @@ bool face_rows_ok(int n_faces, const int32_t* face_to_row, int n_rows)
   return true;
 }
 
-bool sparse_enough(int n_faces, const int32_t* front, const int32_t* rear, const int32_t* face_to_row, int n_rows,
-                   int row_begin, int row_end)
+// What a packed output of rows [row_begin, row_end) may hold.
+struct PairBound {
+  long long pairs = 0;  // a row's nonzero entries are at most min(its rays, n_rows)
+  bool narrow = false;  // a pair fits one word: no column and no count reaches 2^16
+  // sparse enough for the packed transfer: the pairs fit the blocks' caps of a
+  // quarter of their entries.  Denser matrices go dense as a whole.
+  bool sparse = false;
+  size_t pair_bytes() const { return narrow ? sizeof(uint32_t) : sizeof(uint2); }
+};
+
+PairBound pair_bound(int n_faces, const int32_t* front, const int32_t* rear, const int32_t* face_to_row, int n_rows,
+                     int row_begin, int row_end)
 {
   std::vector<long long> rays((size_t)n_rows, 0);
   for (int f = 0; f < n_faces; ++f)
     rays[(size_t)(face_to_row ? face_to_row[f] : f)] += (long long)front[f] + rear[f];
-  long long bound = 0;
+  PairBound b;
   for (int r = row_begin; r < row_end; ++r)
-    bound += std::min<long long>(rays[(size_t)r], n_rows);
-  return bound <= (long long)(row_end - row_begin) * n_rows / 4;
+    b.pairs += std::min<long long>(rays[(size_t)r], n_rows);
+  b.narrow = n_rows <= 65536 && *std::max_element(rays.begin(), rays.end()) < 65536;
+  b.sparse = b.pairs <= (long long)(row_end - row_begin) * n_rows / 4;
+  return b;
 }
 
 // Pinned host memory of at least `bytes` in *p (capacity *cap), kept and
@@ -1211,6 +1226,19 @@ int ensure_pinned(const ffb_ctx* c, uint32_t** p, size_t* cap, size_t bytes)
   FFB_CUDA(cudaMallocHost((void**)p, want));
   *cap = want;
   return FFB_OK;
+}
+
+size_t align256(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// Outputs below FFB_PINNED_MIN_BYTES lock no memory of their own: headers and
+// stages lie in the buffer that the context's uploads go through, whose last
+// copy is ordered before the blocks' traces.  Each stage gets half of what the
+// headers of `rows` rows (in up to 8 blocks) leave.
+size_t small_stage_bytes(const ffb_ctx* c, int rows)
+{
+  const size_t hdr = align256(sizeof(uint32_t) * (2 * (size_t)rows + 8 * 2));
+  const size_t have = std::max(c->pinned_cap, kStageMinBytes);
+  return (have - std::min(have, hdr)) / 2 / 256 * 256;
 }
 
 // A host output of several row blocks moved as (column, count) pairs: called
@@ -1343,9 +1371,18 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   // stream while the next block traces.
   const int span = row_end - row_begin;
   int n_blocks = 1;
+  const bool large = sizeof(uint32_t) * words >= FFB_PINNED_MIN_BYTES;
+  PairBound bound;
   if (host_out && sizeof(uint32_t) * words >= FFB_PIPELINE_MIN_BYTES) {
-    const size_t want = (sizeof(uint32_t) * words + FFB_PIPELINE_BLOCK_BYTES - 1) / FFB_PIPELINE_BLOCK_BYTES;
-    n_blocks = (int)std::min<size_t>(std::max<size_t>(want, 2), (size_t)std::min(kMaxPipeBlocks, span));
+    if (host_threads(c) > 0)
+      bound = pair_bound(s.n_faces, front, rear, face_to_row, n_rows, row_begin, row_end);
+    size_t want = std::max<size_t>((sizeof(uint32_t) * words + FFB_PIPELINE_BLOCK_BYTES - 1) / FFB_PIPELINE_BLOCK_BYTES, 2);
+    // as many as it takes for a block's pairs to fit a stage: 65 MB at one in
+    // four 1.4 ms in five blocks, 3.3 in two of which one went dense
+    if (!large && bound.sparse)
+      while (want < 8 && 2 * bound.pair_bytes() * (size_t)bound.pairs > (2 * want - 1) * small_stage_bytes(c, span))
+        ++want;
+    n_blocks = (int)std::min<size_t>(want, (size_t)std::min(kMaxPipeBlocks, span));
   }
   // Equal blocks, except that the first of several has half the rows (when
   // every block keeps one): the host's side of a pipelined output starts
@@ -1397,31 +1434,16 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   // are enabled and the rows are sparse enough: per block a header
   // (pack_header_words) and at most a quarter of its entries as pairs (at
   // most 1 or 2 bytes per entry with one- or two-word pairs, against 4).
-  bool packed = host_out && n_blocks > 1 && host_threads(c) > 0 &&
-                sparse_enough(s.n_faces, front, rear, face_to_row, n_rows, row_begin, row_end);
+  bool packed = n_blocks > 1 && bound.sparse;
   packed = packed && ensure_host_pool(c);  // without host threads the blocks are copied dense
   if (fs && !packed)
     return fail(FFB_ERR_ARG, "normalised host output without a packed transfer");
-  // One word per pair (column | count << 16) when no column and no count
-  // reaches 2^16: a count is at most its row's rays.
-  bool narrow = false;
-  if (packed && n_rows <= 65536) {
-    std::vector<long long> row_rays(face_to_row ? (size_t)n_rows : 0, 0);
-    long long most = 0;
-    for (int f = 0; f < s.n_faces; ++f) {
-      const long long r = (long long)front[f] + rear[f];
-      if (face_to_row)
-        most = std::max(most, row_rays[(size_t)face_to_row[f]] += r);
-      else
-        most = std::max(most, r);
-    }
-    narrow = most < 65536;
-  }
-  const size_t pair_bytes = narrow ? sizeof(uint32_t) : sizeof(uint2);
+  // One word per pair (column | count << 16), or two.
+  const bool narrow = bound.narrow;
+  const size_t pair_bytes = bound.pair_bytes();
   std::vector<size_t> hdr_off, pair_off;
   std::vector<uint32_t> cap;
   size_t hdr_words = 0, hdr_bytes = 0, stage_bytes = 0;
-  const bool large = sizeof(uint32_t) * words >= (64u << 20);
   c->last_d2h = 0;
   if (packed) {
     size_t& hw = hdr_words;
@@ -1440,19 +1462,21 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
       pw += cap.back();
       max_cap = std::max<size_t>(max_cap, cap.back());
     }
-    // Pinned: the headers and two stages, which hold a block's pairs each.  From
-    // 64 MB on sized at once for blocks of up to FFB_PIPELINE_BLOCK_BYTES (the
-    // blocks of every matrix below 16 of them) and any number of rows.  Locking
-    // memory takes 1.2 ms and 0.2 to 0.3 ms per MB: one block, and a smaller
-    // matrix locks what it needs.
-    hdr_bytes = (std::max(sizeof(uint32_t) * hw, large ? (size_t)1 << 20 : 0) + 255) / 256 * 256;
-    stage_bytes =
-        (std::max(pair_bytes * max_cap, large ? (size_t)FFB_PIPELINE_BLOCK_BYTES / 2 : 0) + 255) / 256 * 256;
+    // Pinned: the headers and two stages, which hold a block's pairs each.
+    hdr_bytes = align256(sizeof(uint32_t) * hw);
     int rc = ensure(c, c->pack_hdr, sizeof(uint32_t) * hw);
     if (rc == FFB_OK)
       rc = ensure(c, c->pack_pairs, pair_bytes * std::max<size_t>(pw, 1));
-    if (rc == FFB_OK)
-      rc = ensure_pinned(c, &c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
+    if (large) {
+      stage_bytes = align256(pair_bytes * max_cap);
+      if (rc == FFB_OK)
+        rc = ensure_pinned(c, &c->pack_host, &c->pack_host_cap, hdr_bytes + 2 * stage_bytes);
+    } else {
+      void* at = c->pinned;
+      if (rc == FFB_OK && !at)
+        rc = stage(c, 1, &at);
+      stage_bytes = small_stage_bytes(c, span);
+    }
     if (rc == FFB_OK && fs) {  // dense blocks are normalised into a device block before their copy
       size_t max_words = 0;
       for (int b = 0; b < n_blocks; ++b)
@@ -1464,9 +1488,11 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
     packed = rc == FFB_OK;  // no room for the pairs: dense blocks
   }
   if (packed) {
-    c->pack_hdr_host = c->pack_host;
+    c->pack_hdr_host = large ? c->pack_host : (uint32_t*)c->pinned;
     for (int k = 0; k < 2; ++k)
-      c->pack_stage[k] = c->pack_host + (hdr_bytes + k * stage_bytes) / sizeof(uint32_t);
+      c->pack_stage[k] = c->pack_hdr_host + (hdr_bytes + k * stage_bytes) / sizeof(uint32_t);
+    for (uint32_t& pairs : cap)
+      pairs = (uint32_t)std::min<size_t>(pairs, stage_bytes / pair_bytes);
   }
   TraceParams p;
   p.frames = dptr<float>(c->frames);
@@ -1732,7 +1758,7 @@ extern "C" int ffb_form_factors(ffb_ctx* c, const int32_t* front, const int32_t*
   FFB_TRY(ptr_kind(c, ff, &ff_dev));
   if (!ff_dev && sizeof(float) * mat >= FFB_PIPELINE_MIN_BYTES && host_threads(c) > 0 && c->main.n_faces > 0 &&
       front && rear && (!face_to_row || face_rows_ok(c->main.n_faces, face_to_row, n_rows)) &&
-      sparse_enough(c->main.n_faces, front, rear, face_to_row, n_rows, 0, n_rows) && ensure_host_pool(c)) {
+      pair_bound(c->main.n_faces, front, rear, face_to_row, n_rows, 0, n_rows).sparse && ensure_host_pool(c)) {
     // a large host matrix: traced in row blocks whose nonzero counts cross
     // PCIe packed and are normalised into the rows by the host threads, with
     // the device's operations: (float)count * (1.f / (float)outgoing[m])
@@ -1744,7 +1770,7 @@ extern "C" int ffb_form_factors(ffb_ctx* c, const int32_t* front, const int32_t*
     bool launched = false;
     const int rc =
         counts_rows_impl(c, front, rear, seed, epoch, flags, face_to_row, n_rows, 0, n_rows, nullptr, &fs, &launched);
-    if (launched || (rc != FFB_ERR_NO_MEMORY && rc != FFB_ERR_CUDA) || sizeof(float) * mat >= (64u << 20))
+    if (launched || (rc != FFB_ERR_NO_MEMORY && rc != FFB_ERR_CUDA) || sizeof(float) * mat >= FFB_PINNED_MIN_BYTES)
       return rc;
     // nothing ran yet, for want of memory (or streams) for the row blocks:
     // dense, in the same memory

@@ -62,3 +62,28 @@ def test_factors_without_room_for_dense_blocks():
     assert np.array_equal(tight.form_factors(front, zero, 9), free.form_factors(front, zero, 9))
     assert tight.device_bytes() - before > 0.4 * matrix  # two dense matrices for one and the pairs
     assert np.array_equal(tight.form_factors(front, zero, 10), free.form_factors(front, zero, 10))
+
+
+@pytest.mark.parametrize("rays", [30, 990, 1024])
+def test_small_outputs_lock_no_memory(rays):
+    """Below 64 MB the pairs go through the upload buffer, in as many row blocks
+    as they need (1024 rays: a quarter of the entries, the most), and a block
+    whose pairs do not fit goes dense (the last rows, with the most rays)."""
+    n = 4096 - 8  # 64 MB less a little
+    faces = np.concatenate([scenes.icosphere(4, 1.0, inward=True)] * 2)[:n]
+    front, zero = np.full(n, rays if rays < 1000 else rays - 3, np.int32), np.zeros(n, np.int32)
+    uneven = np.where(np.arange(n) < 3000, 20, 3 * rays).astype(np.int32)
+    c = native.Context(0)
+    _limit(c, 1)
+    c.scene_set(faces)
+    c.grid_build(cells_per_face=16)
+    for k, f in enumerate((front, uneven)):
+        threads = c.host_threads()
+        got = c.form_factor_counts(f, zero, 5)
+        moved = c.stats().d2h_bytes
+        assert moved < 4 * n * n  # packed, or (the last block) in part
+        assert k or moved < 4 * rays * n + (1 << 20)
+        c.set_host_threads(0)
+        assert np.array_equal(got, c.form_factor_counts(f, zero, 5))
+        assert c.stats().d2h_bytes == 4 * n * n
+        c.set_host_threads(threads)
