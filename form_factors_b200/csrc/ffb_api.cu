@@ -102,6 +102,18 @@ constexpr int kMaxPipeBlocks = 16;  // row blocks of a pipelined host output
 #define FFB_PIPELINE_BLOCK_BYTES (160ull << 20)
 #endif
 
+// Rays of a launch, and the sum of the squares of its faces' rays: over the
+// rays, how many rays share a ray's face on average.
+struct RayTotals {
+  long long rays = 0;
+  double squares = 0.0;
+  void add(long long n)
+  {
+    rays += n;
+    squares += (double)n * (double)n;
+  }
+};
+
 // One resident scene: faces, triangle records and its grid.
 struct SceneData {
   int n_faces = -1;  // -1: no scene
@@ -141,7 +153,7 @@ struct ffb_ctx {
   int batch_frames_mode = -1;
   int batch_n_chunks = 0;
   std::vector<int> batch_chunk_first;  // first chunk of each scene (scene-major), plus the total
-  std::vector<std::pair<long long, long long>> batch_rays;  // rays and emitting faces of each scene
+  std::vector<RayTotals> batch_rays;   // of each scene
   std::vector<int> batch_shape;        // launch shape of each scene (ffb_batch_autotune), default 0
   // side streams of the batched launch: one launch per scene, spread over
   // them so that a scene's launch tail overlaps the next scenes
@@ -364,17 +376,20 @@ GridView make_view(SceneData& s)
 // (parallel plates 5 to 9), up to 6 % slower in those above (clutter).
 int default_shape(const SceneData& s) { return s.info.n_refs < 12ll * s.info.n_live_faces ? 12 : 0; }
 
-// Whether a launch of `rays` rays from `faces` faces reads a scene's test
-// records past the L1 cache (ldg8): when they are larger than it and no face
-// emits so many rays that the whole GPU traces a few faces at a time, whose
-// records then are found in L1 (and, read past it, meet in the same L2 lines).
-// Seven scenes of 1280 to 22 080 faces at two grids each: 500 to 8000 rays per
-// face 1 to 19 % faster past L1, 30 000 from 4 % faster to 26 % slower, 100 000
-// up to 2.2 times slower.  Rays cast from memory stay cached: their order is
-// not known.
-bool stream_records(const SceneData& s, long long rays, long long faces)
+// Whether a launch reads a scene's test records past the L1 cache (ldg8): when
+// they are larger than it and few rays start at faces that emit so many that
+// the whole GPU traces a few faces at a time, whose records then are found in
+// L1 (and, read past it, meet in the same L2 lines).  Seven scenes of 1280 to
+// 22 080 faces at two grids each, equal budgets: 500 to 8000 rays per face 1 to
+// 19 % faster past L1, 30 000 from 4 % faster to 26 % slower, 100 000 up to 2.2
+// times slower; 40 000 at faces far apart 2 to 9 % faster.  20 M rays in the
+// closed room of 22 080 faces at its default grid, of which one face emits all
+// but one per face: 12.4 ms past L1, 6.1 cached; a quarter at five faces 6.0
+// and 5.3, a tenth at two 5.3 both.  Rays cast from memory stay cached: their
+// order is not known.
+bool stream_records(const SceneData& s, const RayTotals& t)
 {
-  return s.info.n_refs * (long long)sizeof(TestRec) >= 256 << 10 && rays <= 10000 * faces;
+  return s.info.n_refs * (long long)sizeof(TestRec) >= 256 << 10 && t.squares <= 10000.0 * (double)t.rays;
 }
 
 int check_ctx(ffb_ctx* c)
@@ -1403,11 +1418,11 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   }
   // emitting faces block after block (ascending within a block)
   std::vector<std::vector<int32_t>> by_block(n_blocks);
-  long long emitted = 0;  // rays of the row range
+  RayTotals emitted;  // of the row range
   for (int f = 0; f < s.n_faces; ++f)
     if (face_block[f] >= 0 && front[f] + (long long)rear[f] > 0) {
       by_block[face_block[f]].push_back(f);
-      emitted += front[f] + (long long)rear[f];
+      emitted.add(front[f] + (long long)rear[f]);
     }
   std::vector<int32_t> order;
   order.reserve((size_t)s.n_faces);
@@ -1419,7 +1434,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   block_pos[n_blocks] = order.size();
   std::vector<long long> face_first;
   long long n_chunks = 0;
-  FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, emitted / n_blocks), face_first, &n_chunks, n_blocks == 1));
+  FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, emitted.rays / n_blocks), face_first, &n_chunks, n_blocks == 1));
   std::vector<int> first(n_blocks + 1, 0);
   for (int b = 0; b <= n_blocks; ++b)
     first[b] = (int)(block_pos[b] < order.size() ? face_first[block_pos[b]] : n_chunks);
@@ -1507,7 +1522,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
   p.span = nullptr;
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
-  p.stream_records = stream_records(s, emitted, (long long)order.size());
+  p.stream_records = stream_records(s, emitted);
   // the kernel adds at row * n_rows + col; the output holds rows from
   // row_begin, so its base is moved back by row_begin rows (only rows of the
   // range are ever written)
@@ -1648,9 +1663,12 @@ int ffb_trace_prepare(ffb_ctx* c, const int32_t* front, const int32_t* rear, uin
   FFB_TRY(ensure_frames(c, flags));
   std::vector<int32_t> order;
   order.reserve((size_t)s.n_faces);
+  RayTotals emitted;
   for (int f = 0; f < s.n_faces; ++f)
-    if (front[f] + (long long)rear[f] > 0)
+    if (front[f] + (long long)rear[f] > 0) {
       order.push_back(f);
+      emitted.add(front[f] + (long long)rear[f]);
+    }
   std::vector<long long> first;
   long long nch = 0;
   FFB_TRY(device_chunks(c, order, front, rear, kChunkRays, first, &nch));
@@ -1675,7 +1693,7 @@ int ffb_trace_prepare(ffb_ctx* c, const int32_t* front, const int32_t* rear, uin
   p.span = dptr<unsigned long long>(c->span);
   p.scene.g = make_view(s);
   p.default_shape = default_shape(s);
-  p.stream_records = stream_records(s, total, (long long)order.size());
+  p.stream_records = stream_records(s, emitted);
   p.scene.counts = counts;
   p.scene.face_to_row = nullptr;
   p.scene.face_base = 0;
@@ -1822,9 +1840,12 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
   FFB_TRY(ensure_frames(c, flags));
   std::vector<int32_t> order;
   order.reserve((size_t)s.n_faces);
+  RayTotals emitted;
   for (int f = 0; f < s.n_faces; ++f)
-    if (front[f] + (long long)rear[f] > 0)
+    if (front[f] + (long long)rear[f] > 0) {
       order.push_back(f);
+      emitted.add(front[f] + (long long)rear[f]);
+    }
   std::vector<long long> face_first;
   long long n_chunks = 0;
   FFB_TRY(device_chunks(c, order, front, rear, chunk_rays(c, total), face_first, &n_chunks, true));
@@ -1862,7 +1883,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
     p.absorb_stride = tally.stride;
     p.span = nullptr;
     p.scene.g = make_view(s);
-    p.stream_records = stream_records(s, total, (long long)order.size());
+    p.stream_records = stream_records(s, emitted);
     p.scene.counts = nullptr;
     p.scene.face_to_row = dptr<int32_t>(c->rows);
     p.scene.face_base = 0;
@@ -1958,7 +1979,7 @@ extern "C" int ffb_parallel_rays(ffb_ctx* c, const ffb_disc_source* src, long lo
   if (n_rays) {
     const GridView g = make_view(s);
     const bool stats = c->stats_on;
-    auto kern = stream_records(s, 0, 0) ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<false, true>)
+    auto kern = stream_records(s, RayTotals{}) ? (stats ? k_parallel_rays<true, true> : k_parallel_rays<false, true>)
                                         : (stats ? k_parallel_rays<true, false> : k_parallel_rays<false, false>);
     int per_sm = 0;
     FFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceThreads, 0));
@@ -2601,7 +2622,7 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
   std::vector<int4> src, tail;
   src.reserve((size_t)n_all);
   c->batch_chunk_first.assign(n_scenes + 1, 0);
-  c->batch_rays.assign(n_scenes, {0, 0});
+  c->batch_rays.assign(n_scenes, RayTotals{});
   long long next = 0;
   for (int s = 0; s < n_scenes; ++s) {
     const long long f0 = c->batch_offsets[s];
@@ -2622,11 +2643,10 @@ extern "C" int ffb_batch_prepare(ffb_ctx* c, const int32_t* front, const int32_t
       (is_tail ? tail : src).push_back(make_int4(f, front[f0 + f], (int)nf, (int)next));
       next += (nf + per - 1) / per;
       rays += nf;
-      ++c->batch_rays[s].second;
+      c->batch_rays[s].add(nf);
       if (next > INT_MAX)
         return fail(FFB_ERR_TOO_LARGE, "more than %d work chunks", INT_MAX);
     }
-    c->batch_rays[s].first = rays;
   }
   c->batch_chunk_first[n_scenes] = (int)next;
   c->batch_n_chunks = (int)next;
@@ -2725,7 +2745,7 @@ extern "C" int ffb_batch_launch(ffb_ctx* c, uint32_t* counts, const unsigned lon
     SceneSlot& slot = p.scene;
     slot.g = make_view(c->batch[s]);
     p.default_shape = default_shape(c->batch[s]);
-    p.stream_records = stream_records(c->batch[s], c->batch_rays[s].first, c->batch_rays[s].second);
+    p.stream_records = stream_records(c->batch[s], c->batch_rays[s]);
     slot.counts = counts + counts_offsets[s];
     slot.face_to_row = nullptr;
     slot.face_base = (int)c->batch_offsets[s];

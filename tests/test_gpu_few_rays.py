@@ -28,3 +28,34 @@ def test_many_chunks_per_fill(ctx, oracle, most, large):
         assert np.array_equal(got, want), "shape %d: %d entries differ" % (shape, (got != want).sum())
     ctx.set_trace_shape(0)
     ctx.set_stats(True)
+
+
+@pytest.mark.parametrize("most", [0, 400000])
+def test_one_face_with_most_rays(ctx, oracle, most):
+    """Budgets far from even (one face emits nearly everything) and even ones take
+    different loads of the test records, larger here than the L1 cache."""
+    faces = scenes.clutter(600, 0.1, seed=5, enclosure_cells=7)
+    n = len(faces)
+    front, zero = np.full(n, 20, np.int32), np.zeros(n, np.int32)
+    front[n // 2] += most
+    ctx.scene_set(faces)
+    ctx.grid_build()
+    assert ctx.grid_info().n_refs * 64 > 256 << 10
+    want = oracle.form_factor_counts(faces, front, zero, seed=3)
+    assert np.array_equal(ctx.form_factor_counts(front, zero, seed=3), want)
+    one = np.ones(n, np.float32)
+    mesh = np.arange(n, dtype=np.int32)
+    got = ctx.radiance_absorption(front, zero, one, one, mesh, n, seed=3)
+    assert np.array_equal(np.rint(got).astype(np.int64), want.sum(0))  # whole numbers: one unit per ray
+    ctx.batch_set([faces], cells_per_face=32)
+    ctx.batch_prepare(front, zero, np.array([3], np.uint64))
+    assert np.array_equal(_batch_counts(ctx, n), want)
+
+
+def _batch_counts(ctx, n):
+    import torch
+    offs, words = ctx.batch_counts_layout()
+    counts = torch.empty(words, dtype=torch.int32, device="cuda")
+    ctx.batch_launch(counts, offs, advance_epoch=False)
+    ctx.synchronize()
+    return counts.cpu().numpy().view(np.uint32)[int(offs[0]):int(offs[0]) + n * n].reshape(n, n)
