@@ -75,6 +75,7 @@ struct DevBuf {
 constexpr int kChunkRays = 256;  // rays per work chunk of the fused kernel at most
 constexpr int kTailRays = 64;    // rays per chunk of a launch's last sixteenth at most
 static_assert(kChunkRays == kChunkRaysMax, "the coherent hand-out orders whole chunks");
+constexpr int kAutoShape = -1;   // launch shape not chosen: the scene's (default_shape)
 constexpr int kMaxRows = 65535;  // matrix index row * n + col stays below 0xFFFFFFFF
 constexpr size_t kStageMinBytes = 8 << 20;  // pinned staging buffer of a context
 constexpr int kMaxPipeBlocks = 16;  // row blocks of a pipelined host output
@@ -141,7 +142,7 @@ struct ffb_ctx {
   unsigned long long budget = 0;  // 0 = unlimited
   unsigned long long bytes = 0;   // device bytes held in DevBufs
   bool stats_on = true;           // fused kernel with counters
-  int trace_shape = 0;            // launch shape of the fused kernel (trace_shape(), chosen by ffb_autotune)
+  int trace_shape = kAutoShape;   // launch shape of the fused kernel (trace_shape(), chosen by ffb_autotune)
 
   SceneData main;                 // the scene of the single-scene calls
   DevBuf frames;                  // emission frames of the main scene
@@ -154,7 +155,7 @@ struct ffb_ctx {
   int batch_n_chunks = 0;
   std::vector<int> batch_chunk_first;  // first chunk of each scene (scene-major), plus the total
   std::vector<RayTotals> batch_rays;   // of each scene
-  std::vector<int> batch_shape;        // launch shape of each scene (ffb_batch_autotune), default 0
+  std::vector<int> batch_shape;        // launch shape of each scene (ffb_batch_autotune), default kAutoShape
   // side streams of the batched launch: one launch per scene, spread over
   // them so that a scene's launch tail overlaps the next scenes
   cudaStream_t batch_streams[4] = {};
@@ -368,12 +369,13 @@ GridView make_view(SceneData& s)
   return g;
 }
 
-// The launch shape that shape 0 stands for in a scene: two references tested
+// The launch shape of a scene where none was chosen: two references tested
 // per iteration, or three where the grid lists fewer than twelve references
 // per face, that is where cells are large against the faces and hold several
-// each.  Three against two on 16 scenes of 64 to 20 480 faces at the default,
-// 64 and 192 cells per face: 0 to 9 % faster in the 18 grids below twelve
-// (parallel plates 5 to 9), up to 6 % slower in those above (clutter).
+// each.  Three against two on 14 scenes of 12 to 22 080 faces at the default,
+// 16, 64 and 192 cells per face: up to 11 % faster in the 26 grids below twelve
+// (parallel plates most), but for three of them with 16 cells per face (1 to 5 %
+// slower); above twelve up to 6 % slower (clutter and the box), at best equal.
 int default_shape(const SceneData& s) { return s.info.n_refs < 12ll * s.info.n_live_faces ? 12 : 0; }
 
 // Whether a launch reads a scene's test records past the L1 cache (ldg8): when
@@ -808,14 +810,10 @@ void (*fused_kernel(const TraceParams& p, bool hash, int shape))(TraceParams)
 
 // Occupancy-sized persistent launch of the fused kernel for p.n_chunks
 // chunks, in the context's launch shape (the counter and radiance variants
-// always take shape 0).
-int launch_fused(ffb_ctx* c, const TraceParams& p, bool timed, cudaStream_t stream = nullptr, int shape = -1)
+// always take shape 0), or `shape`.
+int launch_fused(ffb_ctx* c, const TraceParams& p, bool timed, cudaStream_t stream, int shape)
 {
-  if (!stream)
-    stream = c->stream;
-  if (shape < 0)
-    shape = c->trace_shape;
-  if (shape == 0)
+  if (shape == kAutoShape)
     shape = p.default_shape;
   const bool hash =
       !p.power && (unsigned long long)p.scene.n_cols * (unsigned long long)p.scene.n_cols < FFB_DIRECT_MIN_WORDS;
@@ -1555,7 +1553,7 @@ int counts_rows_impl(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint
         p.chunks = dptr<Chunk>(c->chunks) + first[b];
         p.n_chunks = first[b + 1] - first[b];
         p.chunk_cursor = dptr<uint32_t>(c->cursor) + b;
-        FFB_TRY(launch_fused(c, p, false, st));
+        FFB_TRY(launch_fused(c, p, false, st, c->trace_shape));
       }
       if (packed && bounds[b + 1] > bounds[b]) {
         const int rows = bounds[b + 1] - bounds[b];
@@ -1718,7 +1716,7 @@ int ffb_trace_slice(ffb_ctx* c, long long first, long long count, void* stream)
   // slices of one prepared trace run in stream order, so one cursor serves them all
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   FFB_CUDA(cudaMemsetAsync(p.chunk_cursor, 0, sizeof(uint32_t), st));
-  return launch_fused(c, p, false, st);
+  return launch_fused(c, p, false, st, c->trace_shape);
 }
 
 int ffb_trace_span(ffb_ctx* c, unsigned long long* start_ns, unsigned long long* end_ns)
@@ -1888,7 +1886,7 @@ extern "C" int ffb_radiance_absorption(ffb_ctx* c, const int32_t* front, const i
     p.scene.face_to_row = dptr<int32_t>(c->rows);
     p.scene.face_base = 0;
     p.scene.n_cols = n_meshes;
-    FFB_TRY(launch_fused(c, p, true));
+    FFB_TRY(launch_fused(c, p, true, c->stream, 0));
   }
   if (tally.copies > 1) {
     k_tally_sum<<<(n_meshes + kSumCounters - 1) / kSumCounters, kSumCounters * kSumLanes, 0, c->stream>>>(
@@ -2585,7 +2583,7 @@ extern "C" int ffb_batch_set(ffb_ctx* c, int n_scenes, const long long* face_off
   c->batch_offsets.assign(face_offsets, face_offsets + n_scenes + 1);
   c->batch_frames_mode = -1;
   c->batch_n_chunks = 0;
-  c->batch_shape.assign((size_t)n_scenes, 0);
+  c->batch_shape.assign((size_t)n_scenes, kAutoShape);
   for (int s = 0; s < n_scenes; ++s) {
     const long long f0 = face_offsets[s];
     const int n = (int)(face_offsets[s + 1] - f0);
@@ -2751,7 +2749,7 @@ extern "C" int ffb_batch_launch(ffb_ctx* c, uint32_t* counts, const unsigned lon
     slot.face_base = (int)c->batch_offsets[s];
     slot.n_cols = c->batch[s].n_faces;
     cudaStream_t st = c->batch_streams[k++ % kSide];
-    const int shape = s < (int)c->batch_shape.size() ? c->batch_shape[(size_t)s] : 0;
+    const int shape = s < (int)c->batch_shape.size() ? c->batch_shape[(size_t)s] : kAutoShape;
     FFB_TRY(launch_fused(c, p, false, st, shape));
   }
   for (int j = 0; j < kSide; ++j) {
@@ -2850,7 +2848,16 @@ extern "C" int ffb_ctx_set_trace_shape(ffb_ctx* c, int shape)
   return FFB_OK;
 }
 
-extern "C" int ffb_ctx_trace_shape(ffb_ctx* c) { return c ? c->trace_shape : FFB_ERR_ARG; }
+extern "C" int ffb_ctx_trace_shape(ffb_ctx* c)
+{
+  if (!c)
+    return FFB_ERR_ARG;
+  if (c->trace_shape != kAutoShape)
+    return c->trace_shape;
+  return c->main.grid_ok ? default_shape(c->main) : 0;
+}
+
+void ffb_ctx_auto_trace_shape(ffb_ctx* c) { c->trace_shape = kAutoShape; }
 
 extern "C" int ffb_autotune(ffb_ctx* c, const int32_t* front, const int32_t* rear, uint64_t seed,
                             const ffb_grid_params* candidates, int n_candidates, int sample_every, int flags,
@@ -3009,7 +3016,7 @@ extern "C" int ffb_batch_autotune(ffb_ctx* c, const int32_t* front, const int32_
     return fail(FFB_ERR_NO_SCENE, "no batch set");
   long long total = 0;
   FFB_TRY(check_counts((int)c->batch_offsets[n_scenes], front, rear, &total));
-  c->batch_shape.assign((size_t)n_scenes, 0);
+  c->batch_shape.assign((size_t)n_scenes, kAutoShape);
   for (int i = 0; i < n_scenes; ++i) {
     SceneData& b = c->batch[i];
     const long long f0 = c->batch_offsets[i];

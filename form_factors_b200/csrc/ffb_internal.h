@@ -13,6 +13,10 @@ int ffb_set_error(int code, const char* msg);
 // `bytes` fail as they do on a host that cannot lock so much (0: none fails).
 extern "C" void ffb_test_pinned_limit(ffb_ctx* c, unsigned long long bytes);
 
+// Takes back a chosen launch shape: the context's traces choose by the scene
+// again (ffb_ctx_set_trace_shape).
+void ffb_ctx_auto_trace_shape(ffb_ctx* c);
+
 // Sliced traces, for the serving loop.  ffb_trace_prepare readies one fused
 // form-factor trace of the context's scene (grid built) with per-face
 // (front, rear) ray counts, Philox (seed, epoch) and emission flags: it

@@ -187,9 +187,8 @@ int prepare(Slot& sl, Request& r, long long* n_chunks)
   std::vector<int32_t> front((size_t)r.n_faces, r.rays_per_face), rear((size_t)r.n_faces, 0);
   if (r.cells_per_face > 0) {
     ffb_grid_params gp = {0, 0, 0, r.cells_per_face, 1};
-    rc = ffb_ctx_set_trace_shape(ctx, 0);
-    if (rc >= 0)
-      rc = ffb_grid_build(ctx, &gp);
+    ffb_ctx_auto_trace_shape(ctx);
+    rc = ffb_grid_build(ctx, &gp);
   } else {
     // grid and launch shape from the tuning cache (a tuning run on a miss,
     // with the request's own matrix as the sample's scratch)

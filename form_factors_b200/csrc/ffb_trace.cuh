@@ -68,7 +68,7 @@ struct TraceParams {
   // of the launch, in %globaltimer nanoseconds (atomicMin / atomicMax, so
   // several launches may share one pair)
   unsigned long long* __restrict__ span;
-  int default_shape = 0;        // what launch shape 0 stands for (host only)
+  int default_shape = 0;        // the launch's shape where none was chosen (host only)
   bool stream_records = false;  // test records bypass the L1 cache, see ldg8 (host only)
   SceneSlot scene;
 };
@@ -202,7 +202,7 @@ constexpr int kRefillMin = FFB_REFILL_MIN;
 // iteration, the idle lanes a warp waits for before it refills them, and the
 // resident blocks of 128 threads per SM the kernel is compiled for (which
 // caps its registers at 65536 / (128 * blocks)).  Shape 0 is the default; where
-// a scene's grid lists few references per face it stands for shape 12.
+// a scene's grid lists few references per face, shape 12 (default_shape).
 // The shape changes only the order in which lanes do their work, never a
 // ray's result or the counts.
 // With `coherent` set, a warp hands out the rays of each chunk it takes in

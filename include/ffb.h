@@ -441,9 +441,11 @@ typedef struct {
 
 int ffb_trace_shape_count(void);
 int ffb_trace_shape_get(int shape, ffb_trace_shape* out);
-/* Launch shape of the context's form-factor traces (default 0, which stands
- * for shape 12 in scenes whose grid lists fewer than twelve references per
- * face: three tests per iteration instead of two). */
+/* Launch shape of the context's form-factor traces.  Until one is set (or
+ * tuned) the scene's: shape 0, or where the grid lists fewer than twelve
+ * references per face shape 12, with three tests per iteration instead of two;
+ * ffb_ctx_trace_shape then returns the one that the present scene would take
+ * (0 without a grid). */
 int ffb_ctx_set_trace_shape(ffb_ctx* ctx, int shape);
 int ffb_ctx_trace_shape(ffb_ctx* ctx);
 
