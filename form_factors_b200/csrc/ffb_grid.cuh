@@ -726,7 +726,7 @@ struct Tracer {
   float bx, by, bz;  // current cell, biased
   float jump;        // empty-space distance of the cell - kBias
   float t_stop;      // the walk ends here: the box exit, or the best hit + slack
-  float far;         // error factor of a ray from outside the box (kFar)
+  float far;         // kFar: error factor of a ray from outside the box, negative for a short one
   uint32_t i, en;    // pending references of the current cell
   int face;          // best hit, -1 if none
   int sx, sy, sz;    // signed cell strides
@@ -821,8 +821,11 @@ __device__ __forceinline__ float walk_speed(float d)
 // Sets up the ray o + t dir; false when it misses the grid box (no hit
 // possible).  *t0 gets the distance from o to the point the walk starts at (0
 // inside the box).  kFar: rays may start far outside the box, and their tests
-// widen the error bounds in proportion; otherwise such a ray takes the exact
-// test for every reference.
+// widen the error bounds in proportion, or be given by an end point very near,
+// and then only rejections are left to the fast test; otherwise such a ray takes
+// the exact test for every reference.  2 M rays cast in the closed room of 22 080
+// faces as segments of 1/32 and 1e-5: 0.89 and 1.12 ms, 1.42 and 1.62 with exact
+// tests alone; whole rays 0.80.
 template <bool kFar>
 __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float3 o, float3 dir, float* t0,
                                              uint32_t& n_cells)
@@ -831,9 +834,14 @@ __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float
   const float dd = __fmaf_rn(dir.x, dir.x, __fmaf_rn(dir.y, dir.y, dir.z * dir.z));
   bool exact = false;
   float rd = rsqrt_approx(dd);
-  if (!(dd >= 0.00390625f && dd < 1e30f)) {
-    // shorter than 1/16 (the fast test's bounds do not hold), huge, zero or
-    // not finite: the last two hit nothing
+  T.far = 1.f;
+  if (kFar && dd >= 0x1p-100f && dd < 0.00390625f) {
+    // shorter than 1/16: the exact test's |n.dir| >= 1e-8 is not certain, so it
+    // decides what the fast test does not reject
+    T.far = -1.f;
+  } else if (!(dd >= 0.00390625f && dd < 1e30f)) {
+    // the fast test's bounds do not hold: every test is exact.  Zero or not
+    // finite: hits nothing
     const float m = fmaxf(fmaxf(fabsf(dir.x), fabsf(dir.y)), fabsf(dir.z));
     if (!(m > 0.f && m < INFINITY) || !(dd == dd))
       return false;
@@ -852,7 +860,6 @@ __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float
   T.pd = f3(walk_speed(T.dg.x), walk_speed(T.dg.y), walk_speed(T.dg.z));
   T.iv = f3(rcp_approx(T.pd.x), rcp_approx(T.pd.y), rcp_approx(T.pd.z));
   T.io = f3(-om.x * T.iv.x, -om.y * T.iv.y, -om.z * T.iv.z);
-  T.far = 1.f;
   if (om.x < 0.f || om.y < 0.f || om.z < 0.f) {
     // outside: the walk starts where the ray enters the box
     const float te = fmaxf(fmaxf(T.io.x, T.io.y), T.io.z);
@@ -866,7 +873,7 @@ __device__ __forceinline__ bool tracer_begin(Tracer& T, const GridView& g, float
     T.io = f3(-om.x * T.iv.x, -om.y * T.iv.y, -om.z * T.iv.z);
     *t0 = te;
     if (kFar)
-      T.far = __fmaf_rn(te, g.inv_size, 1.f);
+      T.far *= __fmaf_rn(te, g.inv_size, 1.f);
     else
       exact = true;
   }
@@ -942,14 +949,15 @@ __device__ __forceinline__ int tracer_test(Tracer& T, const GridView& g, uint32_
   const float s = __fmaf_rn(q[6], z, __fmaf_rn(q[5], y, __fmaf_rn(q[4], x, q[7])));
   const float r = __fmaf_rn(q[10], z, __fmaf_rn(q[9], y, __fmaf_rn(q[8], x, q[11])));
   const float m = fminf(fminf(s, r), (1.f - s) - r);
-  const float e = kFar ? fabsf(ib) * T.far : fabsf(ib);
+  const float e = kFar ? fabsf(ib * T.far) : fabsf(ib);
   const float t_lo = __fmaf_rn(-q[13], e, t), t_hi = __fmaf_rn(q[13], e, t);
   if ((m < -e) | (t_hi < 0.f) | (t_lo > T.t_stop))
     return -1;
   const int f = __float_as_int(q[12]);
   if (f == T.face)
     return -1;
-  if (m > e && t_lo > 0.f && t_hi - t < g.near_err && (T.face < 0 || t_hi < T.t_stop - g.tie)) {
+  const bool inside = m > e && (!kFar || T.far > 0.f);
+  if (inside && t_lo > 0.f && t_hi - t < g.near_err && (T.face < 0 || t_hi < T.t_stop - g.tie)) {
     T.face = f;
     T.t_stop = fminf(T.t_stop, t + g.slack);
     return -1;

@@ -3,7 +3,8 @@
 tests/cpp/tracer_check.cpp builds form_factors_b200/csrc/ffb_grid.cuh as plain
 C++ and compares the faces its traversal finds with a scan over every face
 (ray_caster/naive_cpu.cpp:65-97), for rays with direction components from 2^-60
-down to the smallest float, and checks that no ray of scenes from the smallest to
+down to the smallest float and for rays given by end points down to a billionth of
+the scene away, and checks that no ray of scenes from the smallest to
 the largest floats reads outside the cell table.  Once more under the compiler's
 checks of undefined arithmetic: cell indices wrap modulo 2^32.  Tolerance: none."""
 import os
