@@ -362,7 +362,6 @@ GridView make_view(SceneData& s)
   g.near_err = 0.25f * I.margin;
   const TestGeom t = test_geom(I);
   g.inv_size = (float)(1.25 / t.size);
-  g.ref_tri = dptr<int32_t>(s.ref_tri);
   g.ref_rec = dptr<TestRec>(s.ref_rec);
   g.tri = dptr<TriRec>(s.tri);
   g.cell_rec = dptr<uint2>(s.cell_rec) + cell_pad(I.nx, I.ny);
@@ -2834,7 +2833,7 @@ extern "C" int ffb_trace_shape_get(int shape, ffb_trace_shape* out)
   if (shape < 0 || shape >= kNumShapes || !out)
     return fail(FFB_ERR_ARG, "shape %d outside [0, %d)", shape, kNumShapes);
   const TraceShape t = trace_shape(shape);
-  *out = ffb_trace_shape{t.adv, t.test, t.refill, t.blocks, t.coherent, t.lanes};
+  *out = ffb_trace_shape{t.adv, t.test, t.refill, t.blocks, t.coherent, 0};
   return FFB_OK;
 }
 

@@ -133,17 +133,6 @@ __device__ __forceinline__ float dist2(float3 p, float3 o)
   return d.x * d.x + d.y * d.y + d.z * d.z;
 }
 
-// Nearest-hit update equivalent to scanning faces in index order with a
-// strict '<' starting from FLT_MAX: the smallest distance wins and, among
-// equal distances, the lowest index.
-__device__ __forceinline__ void consider(float d, int idx, float& best, int& best_idx)
-{
-  if (d < best || (d == best && idx < best_idx)) {
-    best = d;
-    best_idx = idx;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11), constants as published.
 // ---------------------------------------------------------------------------

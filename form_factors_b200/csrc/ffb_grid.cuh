@@ -43,7 +43,7 @@ struct alignas(32) TestRec {
 };
 
 struct GridView {
-  float3 lo, hi;        // grid box
+  float3 lo;            // grid box, low corner
   float3 inv_cs;        // 1 / cell size
   float3 nf;            // cells per axis
   float3 eps;           // landing bias, cells: a quarter of the margin (at most a quarter of a cell)
@@ -53,7 +53,6 @@ struct GridView {
   float tie;            // slack + margin
   float near_err;       // margin / 4: the largest distance error of a hit accepted without the exact test
   float inv_size;       // 1.25 / box diagonal
-  const int32_t* __restrict__ ref_tri;      // triangle index per reference
   const TestRec* __restrict__ ref_rec;      // test record per reference (a copy of its face's)
   const TriRec* __restrict__ tri;           // exact triangle record per face
   const uint2* __restrict__ cell_rec;       // per cell: {start, end} of its references, or octant distances

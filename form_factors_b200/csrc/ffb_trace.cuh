@@ -209,27 +209,26 @@ constexpr int kRefillMin = FFB_REFILL_MIN;
 // the order of their directions (bins of an 8 x 8 Morton order on the Malley
 // disk) instead of in index order, so that lanes refilled together trace
 // rays of similar direction from the same face.
-// `lanes` (rays per lane kept in shared memory) is 0 in every shape.
 struct TraceShape {
-  int adv, test, refill, blocks, coherent, lanes;
+  int adv, test, refill, blocks, coherent;
 };
 constexpr int kNumShapes = 14;
 __host__ __device__ constexpr TraceShape trace_shape(int v)
 {
-  return v == 1 ? TraceShape{1, 1, 4, 8, 0, 0}
-       : v == 2 ? TraceShape{2, 1, 6, 8, 0, 0}
-       : v == 3 ? TraceShape{1, 2, 6, 8, 0, 0}
-       : v == 4 ? TraceShape{3, 3, 6, 8, 0, 0}
-       : v == 5 ? TraceShape{2, 2, 10, 8, 0, 0}
-       : v == 6 ? TraceShape{2, 2, 6, 6, 0, 0}
-       : v == 7 ? TraceShape{2, 2, 6, 8, 1, 0}
-       : v == 8 ? TraceShape{2, 2, 10, 8, 1, 0}
-       : v == 9 ? TraceShape{2, 2, 8, 7, 0, 0}
-       : v == 10 ? TraceShape{2, 4, 8, 8, 0, 0}
-       : v == 11 ? TraceShape{4, 2, 8, 8, 0, 0}
-       : v == 12 ? TraceShape{2, 3, 8, 8, 0, 0}
-       : v == 13 ? TraceShape{3, 2, 8, 8, 1, 0}
-                 : TraceShape{FFB_ADV_PER_ITER, FFB_TEST_PER_ITER, FFB_REFILL_MIN, FFB_MIN_BLOCKS, 0, 0};
+  return v == 1 ? TraceShape{1, 1, 4, 8, 0}
+       : v == 2 ? TraceShape{2, 1, 6, 8, 0}
+       : v == 3 ? TraceShape{1, 2, 6, 8, 0}
+       : v == 4 ? TraceShape{3, 3, 6, 8, 0}
+       : v == 5 ? TraceShape{2, 2, 10, 8, 0}
+       : v == 6 ? TraceShape{2, 2, 6, 6, 0}
+       : v == 7 ? TraceShape{2, 2, 6, 8, 1}
+       : v == 8 ? TraceShape{2, 2, 10, 8, 1}
+       : v == 9 ? TraceShape{2, 2, 8, 7, 0}
+       : v == 10 ? TraceShape{2, 4, 8, 8, 0}
+       : v == 11 ? TraceShape{4, 2, 8, 8, 0}
+       : v == 12 ? TraceShape{2, 3, 8, 8, 0}
+       : v == 13 ? TraceShape{3, 2, 8, 8, 1}
+                 : TraceShape{FFB_ADV_PER_ITER, FFB_TEST_PER_ITER, FFB_REFILL_MIN, FFB_MIN_BLOCKS, 0};
 }
 
 constexpr int kChunkRaysMax = 256;  // rays per chunk (the host's chunk size)
