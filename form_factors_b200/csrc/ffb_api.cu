@@ -611,7 +611,9 @@ int grid_build(ffb_ctx* c, SceneData& s, const ffb_grid_params* params)
   bg.margin = margin;
   // Lanes per face of the binning: enough to fill the GPU, at most a warp (12
   // faces: 28 -> 4 us, 4028 faces: 17 -> 6 us); the lanes of a face repeat its
-  // set-up, so a scene that fills the GPU by itself takes fewer.
+  // set-up, so a scene that fills the GPU by itself takes fewer (1 M faces of 89
+  // cells, whole build: 20.9 ms; 28.2 with divisions for each cell, 24.8 with
+  // three nested loops).
   int lanes_log2 = 0;
   while (lanes_log2 < 5 && ((long long)s.n_faces << lanes_log2) < 2048ll * c->n_sm)
     ++lanes_log2;

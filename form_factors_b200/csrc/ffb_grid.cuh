@@ -243,9 +243,16 @@ __device__ __forceinline__ void for_each_cell(const BinGeom& g, const float* __r
   const int ni = i1 - i0 + 1, nj = j1 - j0 + 1, count = ni * nj * (k1 - k0 + 1);
   if (ni <= 0 || nj <= 0)
     return;
-  for (int at = lane; at < count; at += lanes) {
-    const int row = at / ni;
-    const int i = i0 + at - row * ni, j = j0 + row % nj, k = k0 + row / nj;
+  const int row = lane / ni;
+  int i = i0 + lane - row * ni, j = j0 + row % nj, k = k0 + row / nj;
+  const auto step = [&] {  // `lanes` cells further; carries instead of divisions
+    for (i += lanes; i > i1; i -= ni)
+      if (++j > j1) {
+        j = j0;
+        ++k;
+      }
+  };
+  for (int at = lane; at < count; at += lanes, step()) {
     if (!flat) {
       float3 c = f3(g.lo.x + ((float)i + 0.5f) * g.cs.x, g.lo.y + ((float)j + 0.5f) * g.cs.y,
                     g.lo.z + ((float)k + 0.5f) * g.cs.z);

@@ -83,6 +83,8 @@ using namespace ffb;
 
 namespace {
 
+long g_binned = 0, g_walks = 0, g_rays = 0, g_bad = 0, g_hits = 0;
+
 struct Scene {
   std::vector<float> faces9;
   std::vector<TriRec> tri;
@@ -185,6 +187,16 @@ Grid make_grid(const Scene& s, int nx, int ny, int nz, bool skip)
   std::vector<std::vector<int>> list((size_t)n_cells);
   for (int f = 0; f < s.n; ++f)
     for_each_cell(bg, s.faces9.data(), f, s.box_lo[f], s.box_hi[f], 0, 1, [&](int c) { list[(size_t)c].push_back(f); });
+  // the cells of a face dealt over the lanes of a group: each once
+  std::vector<int> seen((size_t)n_cells, 0);
+  for (int lanes = 2; lanes <= 32; lanes *= 4)
+    for (int f = 0; f < s.n; ++f) {
+      for (int lane = 0; lane < lanes; ++lane)
+        for_each_cell(bg, s.faces9.data(), f, s.box_lo[f], s.box_hi[f], lane, lanes, [&](int c) { ++seen[(size_t)c]; });
+      for_each_cell(bg, s.faces9.data(), f, s.box_lo[f], s.box_hi[f], 0, 1, [&](int c) { --seen[(size_t)c]; });
+    }
+  for (int n : seen)
+    g_binned += n != 0;
   std::vector<uint32_t> start((size_t)n_cells + 1, 0);
   for (int c = 0; c < n_cells; ++c) {
     start[(size_t)c + 1] = start[(size_t)c] + (uint32_t)list[(size_t)c].size();
@@ -276,8 +288,6 @@ int walk(const Grid& G, float3 o, float3 dir)
     }
   }
 }
-
-long g_walks = 0, g_rays = 0, g_bad = 0, g_hits = 0;
 
 // One ray given by origin and end point, as casts get it.
 void check(const char* what, const Scene& s, const Grid& G, const float* o, const float* e)
@@ -448,6 +458,7 @@ int main()
   small_components();
   short_rays();
   extreme_scales();
-  printf("walks %ld, rays %ld, hits %ld, reads outside the table %ld, mismatches %ld\n", g_walks, g_rays, g_hits, g_outside, g_bad);
-  return g_bad || g_outside || g_hits * 2 < g_rays;
+  printf("cells binned otherwise %ld, walks %ld, rays %ld, hits %ld, reads outside the table %ld, mismatches %ld\n",
+         g_binned, g_walks, g_rays, g_hits, g_outside, g_bad);
+  return g_binned || g_bad || g_outside || g_hits * 2 < g_rays;
 }
