@@ -344,7 +344,10 @@ GridView make_view(SceneData& s)
 {
   GridView g;
   const ffb_grid_info& I = s.info;
-  g.lo = make_float3(I.lo[0], I.lo[1], I.lo[2]);
+  // An extent that overflows has infinite cells: every face and ray is in the
+  // first one along it (0 * (o - lo)), for which the corner has to be finite.
+  const auto corner = [](float lo) { return std::isfinite(lo) ? lo : 0.f; };
+  g.lo = make_float3(corner(I.lo[0]), corner(I.lo[1]), corner(I.lo[2]));
   g.inv_cs = make_float3(1.f / I.cell[0], 1.f / I.cell[1], 1.f / I.cell[2]);
   g.nf = make_float3((float)I.nx, (float)I.ny, (float)I.nz);
   const auto bias = [&](float ics) {
