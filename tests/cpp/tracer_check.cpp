@@ -77,7 +77,18 @@ template <class T> static T atomicAdd(T* p, T v) { const T o = *p; *p += v; retu
 template <class T> static T atomicMin(T* p, T v) { const T o = *p; *p = min(o, v); return o; }
 template <class T> static T atomicMax(T* p, T v) { const T o = *p; *p = max(o, v); return o; }
 
+// A float's conversion to int as the GPU does it: saturating, not a number to 0.
+struct Floor {
+  float v;
+  explicit operator int() const
+  {
+    return v != v ? 0 : v >= 2147483648.f ? INT32_MAX : v < -2147483648.f ? INT32_MIN : (int)v;
+  }
+};
+static Floor floor_gpu(float x) { return {std::floor(x)}; }
+#define floorf floor_gpu
 #include "ffb_grid.cuh"
+#undef floorf
 
 using namespace ffb;
 
@@ -157,7 +168,8 @@ Grid make_grid(const Scene& s, int nx, int ny, int nz, bool skip)
   Grid G;
   GridView& g = G.view;
   memset(&g, 0, sizeof g);
-  g.lo = f3(lo[0], lo[1], lo[2]);
+  const auto corner = [](float x) { return isfinite(x) ? x : 0.f; };
+  g.lo = f3(corner(lo[0]), corner(lo[1]), corner(lo[2]));
   g.inv_cs = f3(1.f / cell[0], 1.f / cell[1], 1.f / cell[2]);
   g.nf = f3((float)nx, (float)ny, (float)nz);
   const auto bias = [&](float ics) {
@@ -176,7 +188,7 @@ Grid make_grid(const Scene& s, int nx, int ny, int nz, bool skip)
   g.inv_size = (float)(1.25 / t.size);
   g.tri = s.tri.data();
   BinGeom bg;
-  bg.lo = g.lo;
+  bg.lo = f3(lo[0], lo[1], lo[2]);
   bg.cs = f3(cell[0], cell[1], cell[2]);
   bg.inv_cs = g.inv_cs;
   bg.nx = nx;
@@ -282,9 +294,9 @@ int walk(const Grid& G, float3 o, float3 dir)
     }
     if (!tracer_advance(T, g, moves, jumps))
       return T.face;
-    if (moves > 4096) {
-      ++g_outside;
-      return -2;
+    if (moves > 1024) {  // at most nx + ny + nz are needed
+      printf("endless walk\n");
+      exit(1);
     }
   }
 }
@@ -422,17 +434,26 @@ void short_rays()
   }
 }
 
-// Scenes from the smallest to the largest floats: no read outside the table,
-// whatever the reference's own arithmetic makes of them.
+// Scenes from the smallest to the largest floats, and two whose extent overflows
+// in some axes or all: no read outside the table and an end to every walk, whatever
+// the reference's own arithmetic makes of them.
 void extreme_scales()
 {
   std::mt19937 rng(12);
   std::uniform_real_distribution<float> u(0.05f, 0.95f);
-  for (int e2 = -140; e2 <= 126; e2 += 7) {
-    const float scale = std::ldexp(1.f, e2);
+  std::vector<int> exponents;
+  for (int e2 = -140; e2 <= 126; e2 += 7)
+    exponents.push_back(e2);
+  exponents.insert(exponents.end(), {127, 1000, 1001});
+  for (const int e2 : exponents) {
+    const float scale = e2 < 1000 ? std::ldexp(1.f, e2) : 1.f;
     const float low[3] = {-0.53f * scale, -0.41f * scale, -0.47f * scale};
-    const Scene s = make_scene(closed_box(scale, 2, low));
-    const int dims[][3] = {{1, 1, 1}, {16, 16, 16}, {256, 2, 3}};
+    std::vector<float> faces = closed_box(scale, 2, low);
+    if (e2 >= 1000)  // a box beside a face too wide for floats
+      for (const float x : {-3e38f, 1.f, 2.f, 3e38f, 2.f, 1.f, 0.f, 3e38f, 3.f})
+        faces.push_back(e2 == 1000 ? x : x > 1e30f || x < -1e30f ? x : -3e38f);
+    const Scene s = make_scene(faces);
+    const int dims[][3] = {{1, 1, 1}, {16, 16, 16}, {8, 8, 8}, {256, 2, 3}};
     for (const auto& d : dims) {
       const Grid G = make_grid(s, d[0], d[1], d[2], true);
       for (int n = 0; n < 1500; ++n) {
@@ -446,6 +467,10 @@ void extreme_scales()
         walk<true>(G, org, v);
         walk<false>(G, org, v);
         ++g_walks;
+        if (e2 >= 1000) {
+          const float e[3] = {o[0] + dir[0], o[1] + dir[1], o[2] + dir[2]};
+          check("overflowing extent", s, G, o, e);
+        }
       }
     }
   }
