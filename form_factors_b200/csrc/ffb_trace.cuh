@@ -179,7 +179,7 @@ __device__ __forceinline__ void warp_hash_flush(uint32_t* keys, uint32_t* vals, 
 //
 // What bounds it: waiting for the loads of cell and test records from L1 and
 // L2, each of which depends on the one before, with the 32 warps per SM that
-// 64 registers leave; then issue (56 % of the slots, 146 warp instructions per
+// 64 registers leave; then issue (58 % of the slots, 146 warp instructions per
 // ray, 14.7 of 32 lanes).  22.08 M rays in the closed room of 22 080 faces at
 // 162^3 cells: 4.61 ms; 4.80 with the records cached in L1 (ldg8), 5.48 with
 // emission by idle lanes and spills in the loop, 9.65 with the exact test for
